@@ -94,9 +94,32 @@ struct BulkSmem {
 __device__ __forceinline__ int ringP(int p) { return (int)((unsigned)(p + 12) % 6u); } // phi: 6 planes
 __device__ __forceinline__ int ringN(int p) { return (int)((unsigned)(p + 3) % 3u); }  // normals: 3 planes
 
-template <int Q, class TF, class TG>
+// PXY: x and y are exact periodic axes (every jet with a nozzle on z, the
+// closed boxes), so that no cell has a ghost layer in x or y; false: either may
+// have one.  Two instantiations because the kernel sits at its 64 registers:
+// with one for both, the branch for x and y ghosts costs the periodic lattices
+// (128 x 128 x 512 jet, D3Q27: FP32 456 -> 465, FP16 424 -> 432 us a launch).
+template <int Q, class TF, class TG, bool PXY = false>
 struct Bulk {
     using A = StepArgs<TF, TG>;
+
+    // PXY folded into the coordinate arithmetic too, for 16-bit f, which is
+    // bound by instruction issue (128 x 128 x 512 jet: D3Q27 FP16 424 -> 409, BF16
+    // 423 -> 410, F16_G32 418 -> 405, D3Q19 FP16 365 -> 348, F16_G32 352 -> 338
+    // us).  FP32 f, bound by load latency, loses by it: the compiler hoists
+    // more out of the plane loop and spills (D3Q27 456 -> 479, D3Q19 379 -> 388).
+    static constexpr bool kConstXY = PXY && sizeof(TF) == 2;
+    static __device__ __forceinline__ bool per_x(const Geometry &G) { return kConstXY || G.bcx == BC_PERIODIC; }
+    static __device__ __forceinline__ bool per_y(const Geometry &G) { return kConstXY || G.bcy == BC_PERIODIC; }
+    // (gx, gy) is a fluid column; with PXY any lattice coordinate is one
+    static __device__ __forceinline__ bool fluid_xy(const Geometry &G, int gx, int gy) {
+        return kConstXY ? gx < (int)G.nx && gy < (int)G.ny
+                   : gx >= G.x_lo && gx <= G.x_hi && gy >= G.y_lo && gy <= G.y_hi;
+    }
+    // the same of a coordinate that halo_axis returned
+    static __device__ __forceinline__ bool fluid_halo(const Geometry &G, int gx, int gy) {
+        return kConstXY || (gx >= G.x_lo && gx <= G.x_hi && gy >= G.y_lo && gy <= G.y_hi);
+    }
 
     // phi^n at fluid cell (x, y, z) with linear index c, from the post-stream
     // phase populations (pull layout: direction q is read at c - c_q).
@@ -166,9 +189,9 @@ struct Bulk {
         const Geometry &G = a.geo;
         int hx, hy;
         phi_border_pos(tid, hx, hy);
-        const int bx = halo_axis(a, x0 - 2 + hx, G.nx, G.bcx == BC_PERIODIC);
-        const int by = halo_axis(a, y0 - 2 + hy, G.ny, G.bcy == BC_PERIODIC);
-        const bool fl = bx >= G.x_lo && bx <= G.x_hi && by >= G.y_lo && by <= G.y_hi;
+        const int bx = halo_axis(a, x0 - 2 + hx, G.nx, per_x(G));
+        const int by = halo_axis(a, y0 - 2 + hy, G.ny, per_y(G));
+        const bool fl = fluid_halo(G, bx, by);
         S.bcell[tid] = fl ? (uint32_t)bx + G.nx * (uint32_t)by : kNoCell;
         S.bpack[tid] = (uint16_t)((hy * kHX + hx) | (bx == 0 ? 1 << 10 : 0) | (bx == (int)G.nx - 1 ? 1 << 11 : 0) |
                                   (by == 0 ? 1 << 12 : 0) | (by == (int)G.ny - 1 ? 1 << 13 : 0));
@@ -204,14 +227,13 @@ struct Bulk {
     // either sum, so their load latencies overlap.
     static __device__ void fill_phi(const A &a, BulkSmem &S, int x0, int y0, int pz, int tid) {
         const Geometry &G = a.geo;
-        const bool px = G.bcx == BC_PERIODIC, py = G.bcy == BC_PERIODIC;
+        const bool px = per_x(G), py = per_y(G);
         const int gz = halo_axis(a, pz, G.nz, G.bcz == BC_PERIODIC);
         const int s = ringP(pz);
         const bool zfluid = gz >= G.z_lo && gz <= G.z_hi; // (gz = -1 outside a non-periodic axis)
-        auto fluid_xy = [&](int gx, int gy) { return gx >= G.x_lo && gx <= G.x_hi && gy >= G.y_lo && gy <= G.y_hi; };
         const int tx = tid % kTX, ty = tid / kTX;
         const int ox = halo_axis(a, x0 + tx, G.nx, px), oy = halo_axis(a, y0 + ty, G.ny, py);
-        const bool fo = zfluid && fluid_xy(ox, oy);
+        const bool fo = zfluid && fluid_halo(G, ox, oy);
         const bool border = tid < kPhiBorder;
         int hx = 0, hy = 0, bx = 0, by = 0;
         if (border) {
@@ -219,7 +241,7 @@ struct Bulk {
             bx = halo_axis(a, x0 - 2 + hx, G.nx, px);
             by = halo_axis(a, y0 - 2 + hy, G.ny, py);
         }
-        const bool fb = border && zfluid && fluid_xy(bx, by);
+        const bool fb = border && zfluid && fluid_halo(G, bx, by);
         float go[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, gb[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         if (fo) gather_g(a, ox, oy, gz, cell_index(G, ox, oy, gz), go);
         if (fb) gather_g(a, bx, by, gz, cell_index(G, bx, by, gz), gb);
@@ -239,7 +261,7 @@ struct Bulk {
                                         int tid) {
         using GB = GBox<TG>;
         const Geometry &G = a.geo;
-        const bool px = G.bcx == BC_PERIODIC, py = G.bcy == BC_PERIODIC;
+        const bool px = per_x(G), py = per_y(G);
         const int gz = halo_axis(a, pz, G.nz, G.bcz == BC_PERIODIC);
         const int s = ringP(pz);
         const bool zfluid = gz >= G.z_lo && gz <= G.z_hi;
@@ -249,7 +271,7 @@ struct Bulk {
             const int gx = halo_axis(a, rx, G.nx, px);
             const int gy = halo_axis(a, ry, G.ny, py);
             float v = 0.f;
-            if (zfluid && gx >= G.x_lo && gx <= G.x_hi && gy >= G.y_lo && gy <= G.y_hi) {
+            if (zfluid && fluid_halo(G, gx, gy)) {
                 const bool edge = (px && (rx < 1 || rx > (int)G.nx - 2)) || (py && (ry < 1 || ry > (int)G.ny - 2));
                 if (edge) {
                     v = phi_from_g(a, gx, gy, gz, cell_index(G, gx, gy, gz));
@@ -300,7 +322,7 @@ struct Bulk {
                                       int tid) {
         const Geometry &G = a.geo;
         const int x = x0 + tx, y = y0 + ty;
-        const bool active = x >= G.x_lo && x <= G.x_hi && y >= G.y_lo && y <= G.y_hi;
+        const bool active = fluid_xy(G, x, y);
         for (int p = zs - 2; p <= zs + 3; ++p) fill_phi(a, S, x0, y0, p, tid);
         if (BORDER_PRE && tid < kPhiBorder) border_setup(a, S, x0, y0, tid); // read back by this thread only
         __syncthreads();
@@ -324,10 +346,10 @@ struct Bulk {
                 const bool more = z + 4 <= ze + 1;
                 const int gz = halo_axis(a, z + 4, G.nz, G.bcz == BC_PERIODIC);
                 const bool zf = gz >= G.z_lo && gz <= G.z_hi;
-                const int ox = halo_axis(a, x, G.nx, G.bcx == BC_PERIODIC);
-                const int oy = halo_axis(a, y, G.ny, G.bcy == BC_PERIODIC);
+                const int ox = halo_axis(a, x, G.nx, per_x(G));
+                const int oy = halo_axis(a, y, G.ny, per_y(G));
                 float go[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                if (more && zf && ox >= G.x_lo && ox <= G.x_hi && oy >= G.y_lo && oy <= G.y_hi)
+                if (more && zf && fluid_halo(G, ox, oy))
                     gather_g(a, ox, oy, gz, cell_index(G, ox, oy, gz), go);
                 if (z + 2 <= ze) fill_nrm_carry(S, z + 2, tid, gc);
                 if (more) {
@@ -346,10 +368,10 @@ struct Bulk {
                     } else if (!BORDER_PRE && tid < kPhiBorder) {
                         int hx, hy;
                         phi_border_pos(tid, hx, hy);
-                        const int bx = halo_axis(a, x0 - 2 + hx, G.nx, G.bcx == BC_PERIODIC);
-                        const int by = halo_axis(a, y0 - 2 + hy, G.ny, G.bcy == BC_PERIODIC);
+                        const int bx = halo_axis(a, x0 - 2 + hx, G.nx, per_x(G));
+                        const int by = halo_axis(a, y0 - 2 + hy, G.ny, per_y(G));
                         float v = 0.f;
-                        if (zf && bx >= G.x_lo && bx <= G.x_hi && by >= G.y_lo && by <= G.y_hi)
+                        if (zf && fluid_halo(G, bx, by))
                             v = phi_from_g(a, bx, by, gz, cell_index(G, bx, by, gz));
                         S.phiZ[sp][hy][hx] = v;
                     }
@@ -395,7 +417,8 @@ struct Bulk {
             gx, gy, gz);
     }
 
-    // The same gradient of the field phi(dx, dy, dz) around the centre.
+    // The same gradient of the field phi(dx, dy, dz) around the centre (the
+    // offsets as integral constants).
     template <class At>
     static __device__ __forceinline__ void grad_at(At &&at, float &gx, float &gy, float &gz) {
         float sx = 0.f, sy = 0.f, sz = 0.f;
@@ -404,7 +427,7 @@ struct Bulk {
             constexpr int cx = cx27(q), cy = cy27(q), cz = cz27(q);
             constexpr float w = (q <= 6) ? VS<Q>::w1 : (q <= 18 ? VS<Q>::w2 : VS<Q>::w3);
             // explicit fused forms: every instantiation rounds alike
-            const float d = at(cx, cy, cz) - at(-cx, -cy, -cz);
+            const float d = at(ic<cx>{}, ic<cy>{}, ic<cz>{}) - at(ic<-cx>{}, ic<-cy>{}, ic<-cz>{});
             if constexpr (cx != 0) sx = fmaf(cx > 0 ? w : -w, d, sx);
             if constexpr (cy != 0) sy = fmaf(cy > 0 ? w : -w, d, sy);
             if constexpr (cz != 0) sz = fmaf(cz > 0 ? w : -w, d, sz);
@@ -645,7 +668,7 @@ struct Bulk {
                                                      const TG *gs = nullptr) {
         const Geometry &G = a.geo;
         const Physics &P = a.phys;
-        const bool px = G.bcx == BC_PERIODIC, py = G.bcy == BC_PERIODIC, pz = G.bcz == BC_PERIODIC;
+        const bool px = per_x(G), py = per_y(G), pz = G.bcz == BC_PERIODIC;
         const uint32_t c0 = cell_index(G, x, y, z);
 
         // (the surface tension from the zeroed-ghost field, phaseField.cuh:246-293,
@@ -676,16 +699,51 @@ struct Bulk {
         if (near_ghost) {
             // phi with ghost values: the ring's for fluid cells, the phi array
             // (written by the boundaries, constant during this kernel) for ghost
-            // cells, 0 outside the lattice
-            auto raw = [&](int dx, int dy, int dz) -> float {
-                const int gx = axis_nb(x + dx, (int)G.nx, px), gy = axis_nb(y + dy, (int)G.ny, py);
-                const int gz = axis_nb(z + dz, (int)G.nz, pz);
-                if (gx < 0 || gy < 0 || gz < 0) return 0.f;
-                if (fluid(G, gx, gy, gz)) return S.phiZ[ringP(z + dz)][hy + dy][hx + dx];
-                return a.fld.phi[cell_index(G, gx, gy, gz)];
-            };
+            // cells
             float gx, gy, gz;
-            grad_at(raw, gx, gy, gz);
+            if constexpr (PXY) {
+                // only the first and last z plane come here
+                grad_at(
+                    [&](auto dx, auto dy, auto dz) -> float {
+                        const int gx = axis_nb(x + dx, (int)G.nx, px), gy = axis_nb(y + dy, (int)G.ny, py);
+                        const int gz = axis_nb(z + dz, (int)G.nz, pz);
+                        if (gx < 0 || gy < 0 || gz < 0) return 0.f;
+                        if (fluid(G, gx, gy, gz)) return S.phiZ[ringP(z + dz)][hy + dy][hx + dx];
+                        return a.fld.phi[cell_index(G, gx, gy, gz)];
+                    },
+                    gx, gy, gz);
+            } else {
+                // With ghost layers in x half of the warps of a lattice ~100 cells
+                // wide come here on every plane.  A fluid cell's neighbours lie
+                // inside the lattice, so which of them are ghosts is six flags,
+                // found once, and a ghost's index is a sum of axis steps; finding
+                // each neighbour's coordinates and testing them against the fluid
+                // range took ~25 instructions a neighbour (101 x 75 x 203 crossflow,
+                // D3Q27, f in half and g in float: 198 us a launch, 138 with the
+                // flags).
+                const bool gxm = !px && x <= G.x_lo, gxp = !px && x >= G.x_hi;
+                const bool gym = !py && y <= G.y_lo, gyp = !py && y >= G.y_hi;
+                const bool gzm = !pz && z <= G.z_lo, gzp = !pz && z >= G.z_hi;
+                // (steps of their own: sharing the gathers' below would keep those
+                // six registers live across this block for every lattice)
+                const uint32_t wxm = px && x == 0 ? G.nx - 1u : 0u - 1u, wxp = px && x == (int)G.nx - 1 ? 1u - G.nx : 1u;
+                const uint32_t wym = py && y == 0 ? G.nxy - G.nx : 0u - G.nx;
+                const uint32_t wyp = py && y == (int)G.ny - 1 ? G.nx - G.nxy : G.nx;
+                const uint32_t wzm = pz && z == 0 ? (uint32_t)G.cells - G.nxy : 0u - G.nxy;
+                const uint32_t wzp = pz && z == (int)G.nz - 1 ? G.nxy - (uint32_t)G.cells : G.nxy;
+                auto flagged = [&](auto cx, auto cy, auto cz) -> float {
+                    constexpr int dx = cx, dy = cy, dz = cz;
+                    float v = S.phiZ[ringP(z + dz)][hy + dy][hx + dx];
+                    bool ghost = false;
+                    uint32_t i = c0;
+                    if constexpr (dx != 0) { ghost |= dx < 0 ? gxm : gxp; i += dx < 0 ? wxm : wxp; }
+                    if constexpr (dy != 0) { ghost |= dy < 0 ? gym : gyp; i += dy < 0 ? wym : wyp; }
+                    if constexpr (dz != 0) { ghost |= dz < 0 ? gzm : gzp; i += dz < 0 ? wzm : wzp; }
+                    if (ghost) v = a.fld.phi[i];
+                    return v;
+                };
+                grad_at(flagged, gx, gy, gz);
+            }
             const float ind = sqrtf(fmaf(gx, gx, fmaf(gy, gy, gz * gz)));
             const float inv = __frcp_rn(ind + 1e-9f);
             nx = gx * inv;
@@ -787,8 +845,8 @@ struct Bulk {
         unroll<0, 7>([&](auto q) { Store<TG>::st(a.gq_dst[q] + c0, go[q]); });
 
         // ---- macroscopic fields needed by the boundaries (or all, on save steps)
-        const bool bplane = (G.bcx == BC_COPY && (x == 1 || x == (int)G.nx - 2)) ||
-                            (G.bcy != BC_PERIODIC && (y == 1 || y == (int)G.ny - 2)) ||
+        const bool bplane = (!kConstXY && G.bcx == BC_COPY && (x == 1 || x == (int)G.nx - 2)) ||
+                            (!kConstXY && G.bcy != BC_PERIODIC && (y == 1 || y == (int)G.ny - 2)) ||
                             (G.bcz != BC_PERIODIC && (z == 1 || z == (int)G.nz - 2));
         if (bplane || (a.flags & 1u)) {
             a.fld.rho[c0] = m.rho;
@@ -803,7 +861,7 @@ struct Bulk {
             a.fld.pxz[c0] = m.pxz;
             a.fld.pyz[c0] = m.pyz;
         }
-        if (a.flags & SSMD_STEP_AVERAGE)
+        if ((a.flags & SSMD_STEP_AVERAGE))
             accumulate_averages(a.avg, c0, (float)(a.status->avg_t + 1u), phi, m.ux, m.uy, m.uz);
         if (!isfinite(m.rho)) atomicOr(&a.status->flags, 1u);
     }
@@ -816,11 +874,12 @@ constexpr uint64_t kTmaWaitNs = 2000000000ull;
 
 // PATH: 1 = per-cell gathers, 2 = TMA boxes for the phi halo, 3 = TMA slabs
 // for the populations (phi halo by gathers).
-template <int Q, class TF, class TG, int PATH>
+// PXY (see Bulk): an instantiation of its own on the gather path.
+template <int Q, class TF, class TG, int PATH, bool PXY = false>
 __global__ void __launch_bounds__(kThreads, PATH == 3 ? 2 : kBulkMinBlocks<Q>)
     bulk_kernel(const StepArgs<TF, TG> a, const __grid_constant__ CUtensorMap gmap,
                 const __grid_constant__ CUtensorMap fmap) {
-    using B = Bulk<Q, TF, TG>;
+    using B = Bulk<Q, TF, TG, PXY>;
     using GB = GBox<TG>;
     __shared__ BulkSmem S;
     const Geometry &G = a.geo;
@@ -836,7 +895,7 @@ __global__ void __launch_bounds__(kThreads, PATH == 3 ? 2 : kBulkMinBlocks<Q>)
     const int zs = G.z_lo + bz * a.zchunk;
     const int ze = min(zs + a.zchunk, G.z_hi + 1);
     const int x = x0 + tx, y = y0 + ty;
-    const bool active = x >= G.x_lo && x <= G.x_hi && y >= G.y_lo && y <= G.y_hi;
+    const bool active = B::fluid_xy(G, x, y);
 
     if constexpr (PATH == 3) {
         extern __shared__ __align__(128) unsigned char dyn3[];

@@ -163,7 +163,7 @@ constexpr size_t bulk_dyn_smem() {
 // Resident bulk work items per SM for this instantiation (queried once per
 // device and kernel, after raising its dynamic shared-memory limit) and the
 // SM count.
-template <int Q, class T, int PATH>
+template <int Q, class T, int PATH, bool PXY = false>
 inline void bulk_slots(int &per_sm, int &sms) {
     static thread_local int cached_dev = -1, cached_per_sm = 0, cached_sms = 0;
     int dev = 0;
@@ -172,9 +172,9 @@ inline void bulk_slots(int &per_sm, int &sms) {
         int n = 0, m = 0;
         const size_t dyn = bulk_dyn_smem<Q, T, PATH>();
         if (dyn > 0)
-            cudaFuncSetAttribute(bulk_kernel<Q, T, phase_t<T>, PATH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(bulk_kernel<Q, T, phase_t<T>, PATH, PXY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)dyn);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bulk_kernel<Q, T, phase_t<T>, PATH>, kThreads, dyn) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bulk_kernel<Q, T, phase_t<T>, PATH, PXY>, kThreads, dyn) !=
             cudaSuccess)
             n = 1;
         if (cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) m = 148;
@@ -288,11 +288,13 @@ int launch_step(const ssmd_params &p, const LBMFields &fl, uint64_t step, uint32
         !(encode_populations<TG>(&gmap, a.g_src, a.geo.nx, a.geo.ny, a.geo.nz, 7, Slab<TG>::WX, kTY) &&
           encode_populations<T>(&fmap, a.f_src, a.geo.nx, a.geo.ny, a.geo.nz, Q, Slab<T>::WX, kTY)))
         return fail(SSMD_ERR_UNSUPPORTED, "slab path needs nx * element size to be a multiple of 16 bytes");
+    const bool pxy = a.geo.bcx == BC_PERIODIC && a.geo.bcy == BC_PERIODIC;
     int per_sm = 1, sms = 1;
     if (path == SSMD_PATH_TMA) bulk_slots<Q, T, 2>(per_sm, sms);
     else if (path == SSMD_PATH_SLAB) {
         if constexpr (kSlabs) bulk_slots<Q, T, 3>(per_sm, sms);
-    } else bulk_slots<Q, T, 1>(per_sm, sms);
+    } else if (pxy) bulk_slots<Q, T, 1, true>(per_sm, sms);
+    else bulk_slots<Q, T, 1>(per_sm, sms);
     tiling(p, a.geo, per_sm * sms, a.tiles_x, a.tiles_y, a.zchunk, a.nzchunks);
     a.halo_mod = (a.geo.bcx == BC_PERIODIC && a.geo.nx < (uint32_t)(kTX + 4)) ||
                  (a.geo.bcy == BC_PERIODIC && a.geo.ny < (uint32_t)(kTY + 4)) ||
@@ -307,7 +309,9 @@ int launch_step(const ssmd_params &p, const LBMFields &fl, uint64_t step, uint32
         bulk_kernel<Q, T, TG, 2><<<nblk, blk, bulk_dyn_smem<Q, T, 2>(), st>>>(a, gmap, fmap);
     else if (path == SSMD_PATH_SLAB) {
         if constexpr (kSlabs) bulk_kernel<Q, T, TG, 3><<<nblk, blk, bulk_dyn_smem<Q, T, 3>(), st>>>(a, gmap, fmap);
-    } else
+    } else if (pxy)
+        bulk_kernel<Q, T, TG, 1, true><<<nblk, blk, 0, st>>>(a, gmap, fmap);
+    else
         bulk_kernel<Q, T, TG, 1><<<nblk, blk, 0, st>>>(a, gmap, fmap);
     if (ev1) cudaEventRecord(ev1, st);
     if (int e = cuda_check(cudaGetLastError(), "bulk_kernel launch")) return e;
