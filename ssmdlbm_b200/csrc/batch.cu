@@ -14,15 +14,24 @@ namespace {
 
 constexpr int kMaxBatch = 4096;
 
+// Whether a batch takes the kernel for lattices periodic in x and y.
+template <class T>
+bool batch_pxy(const ssmd_params *params, int32_t count) {
+    if (sizeof(T) != 2) return false;
+    for (int32_t i = 0; i < count; ++i)
+        if (params[i].bc_x != SSMD_BC_PERIODIC || params[i].bc_y != SSMD_BC_PERIODIC) return false;
+    return true;
+}
+
 // Resident blocks of the batched bulk kernel per SM, and the SM count.
-template <int Q, class T>
+template <int Q, class T, bool PXY = false>
 void batch_slots(int &per_sm, int &sms) {
     static thread_local int dev_cached = -1, n_cached = 1, m_cached = 148;
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev != dev_cached) {
         int n = 0, m = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bulk_batch_kernel<Q, T>, kThreads, 0) != cudaSuccess) n = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bulk_batch_kernel<Q, T, PXY>, kThreads, 0) != cudaSuccess) n = 1;
         if (cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) m = 148;
         dev_cached = dev;
         n_cached = n > 0 ? n : 1;
@@ -105,8 +114,12 @@ int step(const ssmd_params *params, int32_t count, uint64_t step_index, uint32_t
     auto *hdr = static_cast<BatchHeader *>(table);
     auto *inst = reinterpret_cast<BatchInst<T> *>(static_cast<char *>(table) + sizeof(BatchHeader));
     const int parity = (int)(step_index & 1ull);
+    const bool pxy = batch_pxy<T>(params, count);
     int per_sm = 1, sms = 1;
-    batch_slots<Q, T>(per_sm, sms);
+    if constexpr (sizeof(T) == 2) {
+        if (pxy) batch_slots<Q, T, true>(per_sm, sms);
+    }
+    if (!pxy) batch_slots<Q, T>(per_sm, sms);
     uint32_t max_n[3] = {0, 0, 0};
     bool jet_y = false, jet_z = false, copy_x = false, copy_y = false;
     for (int32_t i = 0; i < count; ++i) {
@@ -119,7 +132,10 @@ int step(const ssmd_params *params, int32_t count, uint64_t step_index, uint32_t
         copy_x |= p.bc_x == SSMD_BC_PERIODIC_COPY;
         copy_y |= p.bc_y == SSMD_BC_PERIODIC_COPY;
     }
-    bulk_batch_kernel<Q, T><<<(unsigned)(per_sm * sms), dim3(kTX, kTY), 0, st>>>(hdr, inst, parity, flags);
+    if constexpr (sizeof(T) == 2) {
+        if (pxy) bulk_batch_kernel<Q, T, true><<<(unsigned)(per_sm * sms), dim3(kTX, kTY), 0, st>>>(hdr, inst, parity, flags);
+    }
+    if (!pxy) bulk_batch_kernel<Q, T><<<(unsigned)(per_sm * sms), dim3(kTX, kTY), 0, st>>>(hdr, inst, parity, flags);
     if (int e = cuda_check(cudaGetLastError(), "batched bulk launch")) return e;
     // one launch per boundary kind that some lattice uses, in the single-lattice order
     const dim3 b2(32, 4);

@@ -108,6 +108,12 @@ struct Bulk {
     // 423 -> 410, F16_G32 418 -> 405, D3Q19 FP16 365 -> 348, F16_G32 352 -> 338
     // us).  FP32 f, bound by load latency, loses by it: the compiler hoists
     // more out of the plane loop and spills (D3Q27 456 -> 479, D3Q19 379 -> 388).
+    // the prologue's phi planes two at a time (fill_phi_pair): shorter for the
+    // short columns of small lattices (64 x 64 x 128 jet, D3Q19 FP32: 42.7 -> 41.0
+    // us a step; 101 x 75 x 203 crossflow, D3Q27 F16_G32: 181 -> 177); off where
+    // the plane loop that follows it compiles to the slower code (128 x 128 x 512
+    // jet, D3Q27 with it: BF16 412 -> 421, F16_G32 408 -> 416, FP32 462 -> 465)
+    static constexpr bool kPairPrologue = Q == 19 || !PXY;
     static constexpr bool kConstXY = PXY && sizeof(TF) == 2;
     static __device__ __forceinline__ bool per_x(const Geometry &G) { return kConstXY || G.bcx == BC_PERIODIC; }
     static __device__ __forceinline__ bool per_y(const Geometry &G) { return kConstXY || G.bcy == BC_PERIODIC; }
@@ -249,6 +255,32 @@ struct Bulk {
         if (border) S.phiZ[s][hy][hx] = (((((gb[0] + gb[1]) + gb[2]) + gb[3]) + gb[4]) + gb[5]) + gb[6];
     }
 
+    // Two planes at once (the gather path's prologue, after border_setup): the 28
+    // loads of both planes' own and border elements are in flight together.
+    // A block's prologue is a chain of such round trips to L2 or DRAM before its
+    // first cell; plane by plane it took six of them.
+    static __device__ __forceinline__ void fill_phi_pair(const A &a, BulkSmem &S, int ox, int oy, int pz, int tid) {
+        const Geometry &G = a.geo;
+        const int tx = tid % kTX, ty = tid / kTX;
+        const bool own = fluid_halo(G, ox, oy);
+        const bool border = tid < kPhiBorder;
+        const uint32_t bc = border ? S.bcell[tid] : kNoCell, pk = border ? S.bpack[tid] : 0u;
+        float go[2][7] = {}, gb[2][7] = {};
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int gz = halo_axis(a, pz + k, G.nz, G.bcz == BC_PERIODIC);
+            const bool zf = gz >= G.z_lo && gz <= G.z_hi;
+            if (zf && own) gather_g(a, ox, oy, gz, cell_index(G, ox, oy, gz), go[k]);
+            if (zf && bc != kNoCell) border_gather(a, bc + (uint32_t)gz * G.nxy, pk, gz, gb[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int s = ringP(pz + k);
+            S.phiZ[s][ty + 2][tx + 2] = sum7(go[k]);
+            if (border) (&S.phiZ[s][0][0])[pk & 0x3FFu] = sum7(gb[k]);
+        }
+    }
+
     static __device__ __forceinline__ float tofloat(float v) { return v; }
     static __device__ __forceinline__ float tofloat(__half v) { return __half2float(v); }
     static __device__ __forceinline__ float tofloat(half_g32 v) { return __half2float(v.h); }
@@ -311,20 +343,25 @@ struct Bulk {
     // later iterations read; the ring slots they overwrite (z - 1, z - 2)
     // were last read before the previous barrier, so the gathers of the
     // cell update and the stencil arithmetic of the fills interleave freely.
-    // Ends with a block-wide barrier.  BORDER_PRE: the phi ring's border
-    // element from its sources found once per work item (border_setup);
-    // otherwise found on every plane, which the batched kernel keeps (its
-    // extra live state spills more with the precompute: 18 872 against
-    // 19 590 MLUPS on the 48-lattice sweep, measured back to back).  Both
-    // give the same bits.
-    template <bool BORDER_PRE = true>
+    // Ends with a block-wide barrier.  The phi ring's border element comes from
+    // its sources found once per work item (border_setup).
     static __device__ void run_gather(const A &a, BulkSmem &S, int x0, int y0, int zs, int ze, int tx, int ty,
                                       int tid) {
         const Geometry &G = a.geo;
         const int x = x0 + tx, y = y0 + ty;
         const bool active = fluid_xy(G, x, y);
-        for (int p = zs - 2; p <= zs + 3; ++p) fill_phi(a, S, x0, y0, p, tid);
-        if (BORDER_PRE && tid < kPhiBorder) border_setup(a, S, x0, y0, tid); // read back by this thread only
+        if constexpr (kPairPrologue) {
+            if (tid < kPhiBorder) border_setup(a, S, x0, y0, tid); // read back by this thread only
+            // (the empty asm keeps these from staying live through the plane loop,
+            // which finds its own)
+            int xs = x, ys = y;
+            asm volatile("" : "+r"(xs), "+r"(ys));
+            const int ox = halo_axis(a, xs, G.nx, per_x(G)), oy = halo_axis(a, ys, G.ny, per_y(G));
+            for (int p = zs - 2; p <= zs + 3; p += 2) fill_phi_pair(a, S, ox, oy, p, tid);
+        } else {
+            for (int p = zs - 2; p <= zs + 3; ++p) fill_phi(a, S, x0, y0, p, tid);
+            if (tid < kPhiBorder) border_setup(a, S, x0, y0, tid); // read back by this thread only
+        }
         __syncthreads();
         GradCarry gc(S, tid);
         gc.start(S.phiZ[ringP(zs - 2)], S.phiZ[ringP(zs - 1)], tx + 2, ty + 2);
@@ -351,30 +388,22 @@ struct Bulk {
                 float go[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
                 if (more && zf && fluid_halo(G, ox, oy))
                     gather_g(a, ox, oy, gz, cell_index(G, ox, oy, gz), go);
+                // the border element's gathers too, its cell and wraps from
+                // border_setup (after the normals they were a second exposed
+                // round trip on every plane: 128 x 128 x 512 jet, D3Q19 FP32 381 ->
+                // 373 us, F16_G32 340 -> 335, D3Q27 F16_G32 413 -> 408)
+                float gb[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                uint32_t pk = 0;
+                if (more && tid < kPhiBorder) {
+                    const uint32_t c = S.bcell[tid];
+                    pk = S.bpack[tid];
+                    if (zf && c != kNoCell) border_gather(a, c + (uint32_t)gz * G.nxy, pk, gz, gb);
+                }
                 if (z + 2 <= ze) fill_nrm_carry(S, z + 2, tid, gc);
                 if (more) {
                     const int sp = ringP(z + 4);
                     S.phiZ[sp][ty + 2][tx + 2] = sum7(go);
-                    if (BORDER_PRE && tid < kPhiBorder) {
-                        // the border element: its cell and wraps from border_setup
-                        const uint32_t c = S.bcell[tid], pk = S.bpack[tid];
-                        float v = 0.f;
-                        if (zf && c != kNoCell) {
-                            float gb[7];
-                            border_gather(a, c + (uint32_t)gz * G.nxy, pk, gz, gb);
-                            v = sum7(gb);
-                        }
-                        (&S.phiZ[sp][0][0])[pk & 0x3FFu] = v;
-                    } else if (!BORDER_PRE && tid < kPhiBorder) {
-                        int hx, hy;
-                        phi_border_pos(tid, hx, hy);
-                        const int bx = halo_axis(a, x0 - 2 + hx, G.nx, per_x(G));
-                        const int by = halo_axis(a, y0 - 2 + hy, G.ny, per_y(G));
-                        float v = 0.f;
-                        if (zf && fluid_halo(G, bx, by))
-                            v = phi_from_g(a, bx, by, gz, cell_index(G, bx, by, gz));
-                        S.phiZ[sp][hy][hx] = v;
-                    }
+                    if (tid < kPhiBorder) (&S.phiZ[sp][0][0])[pk & 0x3FFu] = sum7(gb);
                 }
             }
             __syncthreads();
