@@ -138,16 +138,14 @@ int step(const ssmd_params *params, int32_t count, uint64_t step_index, uint32_t
     if (!pxy) bulk_batch_kernel<Q, T><<<(unsigned)(per_sm * sms), dim3(kTX, kTY), 0, st>>>(hdr, inst, parity, flags);
     if (int e = cuda_check(cudaGetLastError(), "batched bulk launch")) return e;
     // one launch per boundary kind that some lattice uses, in the single-lattice order
-    const dim3 b2(32, 4);
-    auto grid = [&](uint32_t n0, uint32_t n1) {
-        return dim3((n0 + 31) / 32, (n1 + 3) / 4, (unsigned)count);
+    auto faces = [&](auto kind, uint32_t n0, uint32_t n1) {
+        constexpr int K = decltype(kind)::value;
+        bc_batch_kernel<Q, T, K><<<face_grid<Q, K>(n0, n1, (unsigned)count), dim3(kFaceX, kFaceY), 0, st>>>(inst, parity);
     };
-    if (jet_y) bc_batch_kernel<Q, T, BK_WATER_IN><<<grid(max_n[0], max_n[2]), b2, 0, st>>>(inst, parity);
-    if (jet_z) bc_batch_kernel<Q, T, BK_OIL_IN><<<grid(max_n[0], max_n[1]), b2, 0, st>>>(inst, parity);
-    if (jet_y) bc_batch_kernel<Q, T, BK_OUT_Y><<<grid(max_n[0], max_n[2]), b2, 0, st>>>(inst, parity);
-    if (jet_z) bc_batch_kernel<Q, T, BK_OUT_Z><<<grid(max_n[0], max_n[1]), b2, 0, st>>>(inst, parity);
-    if (copy_x) bc_batch_kernel<Q, T, BK_COPY_X><<<grid(max_n[1], max_n[2]), b2, 0, st>>>(inst, parity);
-    if (copy_y) bc_batch_kernel<Q, T, BK_COPY_Y><<<grid(max_n[0], max_n[2]), b2, 0, st>>>(inst, parity);
+    if (jet_y) faces(ic<BK_JET_Y>{}, max_n[0], max_n[2]);
+    if (jet_z) faces(ic<BK_JET_Z>{}, max_n[0], max_n[1]);
+    if (copy_x) faces(ic<BK_COPY_X>{}, max_n[1], max_n[2]);
+    if (copy_y) faces(ic<BK_COPY_Y>{}, max_n[0], max_n[2]);
     return cuda_check(cudaGetLastError(), "batched boundary launch");
 }
 

@@ -94,20 +94,10 @@ __global__ void __launch_bounds__(kThreads, kBulkMinBlocks<Q>)
     }
 }
 
-// Boundary kind K of every instance: thread (i0, i1) of face plane, blockIdx.z = instance.
-enum : int { BK_WATER_IN = 0, BK_OIL_IN, BK_OUT_Y, BK_OUT_Z, BK_COPY_X, BK_COPY_Y };
-
+// Boundary kind K (BK_*) of every instance, blockIdx.z = instance.
 template <int Q, class T, int K>
-__global__ void bc_batch_kernel(const BatchInst<T> *inst, int parity) {
-    const StepArgs<T, phase_t<T>> &a = inst[blockIdx.z].args[parity];
-    const int i0 = threadIdx.x + blockIdx.x * blockDim.x, i1 = threadIdx.y + blockIdx.y * blockDim.y;
-    const Geometry &G = a.geo;
-    if constexpr (K == BK_WATER_IN) { if (G.bcy == BC_JET) bc_water_inflow_at<Q>(a, i0, i1); }
-    if constexpr (K == BK_OIL_IN) { if (G.bcz == BC_JET) bc_oil_inflow_at<Q>(a, i0, i1); }
-    if constexpr (K == BK_OUT_Y) { if (G.bcy == BC_JET) bc_outflow_y_at<Q>(a, i0, i1); }
-    if constexpr (K == BK_OUT_Z) { if (G.bcz == BC_JET) bc_outflow_z_at<Q>(a, i0, i1); }
-    if constexpr (K == BK_COPY_X) { if (G.bcx == BC_COPY) bc_copy_x_at<Q>(a, i0, i1); }
-    if constexpr (K == BK_COPY_Y) { if (G.bcy == BC_COPY) bc_copy_y_at<Q>(a, i0, i1); }
+__global__ void __launch_bounds__(kFaceX * kFaceY) bc_batch_kernel(const BatchInst<T> *inst, int parity) {
+    bc_face<Q, K>(inst[blockIdx.z].args[parity]);
 }
 
 } // namespace ssmd

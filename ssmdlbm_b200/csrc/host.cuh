@@ -317,23 +317,14 @@ int launch_step(const ssmd_params &p, const LBMFields &fl, uint64_t step, uint32
     if (int e = cuda_check(cudaGetLastError(), "bulk_kernel launch")) return e;
 
     const Geometry &G = a.geo;
-    const dim3 b2(32, 4);
-    auto grid2 = [&](uint32_t n0, uint32_t n1) {
-        return dim3((n0 + b2.x - 1) / b2.x, (n1 + b2.y - 1) / b2.y);
+    auto faces = [&](auto kind, uint32_t n0, uint32_t n1) {
+        constexpr int K = decltype(kind)::value;
+        bc_kernel<Q, T, TG, K><<<face_grid<Q, K>(n0, n1), dim3(kFaceX, kFaceY), 0, st>>>(a);
     };
-    if (G.bcz == BC_JET && G.bcy != BC_JET && G.nz >= 3) {
-        // the two z faces are independent: one launch (reference order otherwise)
-        dim3 g = grid2(G.nx, G.ny);
-        g.z = 2;
-        bc_jet_z<Q, T, TG><<<g, b2, 0, st>>>(a);
-    } else {
-        if (G.bcy == BC_JET) bc_water_inflow<Q, T, TG><<<grid2(G.nx, G.nz), b2, 0, st>>>(a);
-        if (G.bcz == BC_JET) bc_oil_inflow<Q, T, TG><<<grid2(G.nx, G.ny), b2, 0, st>>>(a);
-        if (G.bcy == BC_JET) bc_outflow_y<Q, T, TG><<<grid2(G.nx, G.nz), b2, 0, st>>>(a);
-        if (G.bcz == BC_JET) bc_outflow_z<Q, T, TG><<<grid2(G.nx, G.ny), b2, 0, st>>>(a);
-    }
-    if (G.bcx == BC_COPY) bc_copy_x<Q, T, TG><<<grid2(G.ny, G.nz), b2, 0, st>>>(a);
-    if (G.bcy == BC_COPY) bc_copy_y<Q, T, TG><<<grid2(G.nx, G.nz), b2, 0, st>>>(a);
+    if (G.bcy == BC_JET) faces(ic<BK_JET_Y>{}, G.nx, G.nz);
+    if (G.bcz == BC_JET) faces(ic<BK_JET_Z>{}, G.nx, G.ny);
+    if (G.bcx == BC_COPY) faces(ic<BK_COPY_X>{}, G.ny, G.nz);
+    if (G.bcy == BC_COPY) faces(ic<BK_COPY_Y>{}, G.nx, G.nz);
     if (flags & SSMD_STEP_AVERAGE) {
         // the bulk kernel updated the fluid cells; the ghost layers follow, then t advances
         const unsigned nb = (unsigned)((G.cells + 255) / 256);

@@ -22,8 +22,10 @@
 
 #if defined(__CUDACC__)
 #define SSMD_HD __host__ __device__ __forceinline__
+#define SSMD_UNROLL _Pragma("unroll")
 #else
 #define SSMD_HD static inline
+#define SSMD_UNROLL
 #endif
 
 namespace ssmd_noise {
@@ -88,6 +90,25 @@ SSMD_HD double dfrombits(int64_t b) {
 }
 #endif
 
+// The series' coefficients, divided and multiplied out by the compiler (IEEE
+// round to nearest, the bits the functions below would get at run time): an
+// inlet cell's 37 dependent FP64 divisions were most of the boundary launch
+// that draws the noise.
+struct Coefficients {
+    double odd[13];        // 1 / (2 i + 1), i = 0 .. 12
+    double rc[12], rs[12]; // signed reciprocal factorials (-1)^n / (2n)!, (-1)^n / (2n + 1)!
+    constexpr Coefficients() : odd(), rc(), rs() {
+        for (int i = 0; i < 13; ++i) odd[i] = 1.0 / (double)(2 * i + 1);
+        double fact = 1.0; // (2n)!
+        for (int n = 0; n < 12; ++n) {
+            if (n > 0) fact = fact * ((double)(2 * n - 1) * (double)(2 * n));
+            const double sign = (n & 1) ? -1.0 : 1.0;
+            rc[n] = sign / fact;
+            rs[n] = sign / (fact * (double)(2 * n + 1));
+        }
+    }
+};
+
 // Natural log for normal positive x: x = m 2^e, m in [sqrt(1/2), sqrt(2)),
 // ln m = 2 atanh(s), s = (m - 1)/(m + 1), |s| < 0.172, series to s^25.
 SSMD_HD double ln(double x) {
@@ -101,8 +122,10 @@ SSMD_HD double ln(double x) {
     }
     const double s = ddiv(dadd(m, -1.0), dadd(m, 1.0));
     const double s2 = dmul(s, s);
+    constexpr Coefficients K{};
     double sum = 0.0;
-    for (int k = 25; k >= 1; k -= 2) sum = dadd(dmul(sum, s2), ddiv(1.0, (double)k));
+    SSMD_UNROLL
+    for (int i = 12; i >= 0; --i) sum = dadd(dmul(sum, s2), K.odd[i]);
     const double lnm = dmul(2.0, dmul(s, sum));
     return dadd(dmul((double)e, 0.69314718055994530942), lnm);
 }
@@ -116,18 +139,12 @@ SSMD_HD double cos_turns(double t) {
     const double a = dmul(r, 6.28318530717958647692);
     const double a2 = dmul(a, a);
     // cos a = sum (-1)^n a^(2n) / (2n)!, sin a = a sum (-1)^n a^(2n) / (2n+1)!
-    double rc[12], rs[12]; // signed reciprocal factorials
-    double fact = 1.0;     // (2n)!
-    for (int n = 0; n < 12; ++n) {
-        if (n > 0) fact = dmul(fact, dmul((double)(2 * n - 1), (double)(2 * n)));
-        const double sign = (n & 1) ? -1.0 : 1.0;
-        rc[n] = ddiv(sign, fact);
-        rs[n] = ddiv(sign, dmul(fact, (double)(2 * n + 1)));
-    }
+    constexpr Coefficients K{};
     double c = 0.0, s = 0.0;
+    SSMD_UNROLL
     for (int n = 11; n >= 0; --n) {
-        c = dadd(dmul(c, a2), rc[n]);
-        s = dadd(dmul(s, a2), rs[n]);
+        c = dadd(dmul(c, a2), K.rc[n]);
+        s = dadd(dmul(s, a2), K.rs[n]);
     }
     s = dmul(s, a);
     switch (((int64_t)k) & 3) {
