@@ -91,7 +91,7 @@ int prepare(const ssmd_params *params, const LBMFields *fields, int32_t count, v
             // different lattices comparable in work
             ssmd_params q = p;
             if (q.tile_z == 0) q.tile_z = 16;
-            tiling(q, a.geo, per_sm * sms, a.tiles_x, a.tiles_y, a.zchunk, a.nzchunks);
+            tiling(q, a.geo, per_sm * sms, sms, a.tiles_x, a.tiles_y, a.zchunk, a.nzchunks);
             a.halo_mod = (a.geo.bcx == BC_PERIODIC && a.geo.nx < (uint32_t)(kTX + 4)) ||
                          (a.geo.bcy == BC_PERIODIC && a.geo.ny < (uint32_t)(kTY + 4)) ||
                          (a.geo.bcz == BC_PERIODIC && a.geo.nz < 6u);

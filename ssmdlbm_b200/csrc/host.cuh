@@ -213,11 +213,38 @@ inline double chunk_makespan(long cols, int nzf, int zc, int slots) {
     return end;
 }
 
+// Small lattices, whose 8-plane chunks do not even fill two resident items per SM:
+// an item's time is then the latency of its planes, about the same alone and
+// with one more item beside it (measured: 1.0 and 1.2-1.3 per plane), so shorter
+// chunks win until there are two per SM.  Chosen: the chunk of 2 .. 8 planes
+// with at most two items per SM whose (planes + prologue) x that factor is least.  B200, us
+// a step alone / among three lattices on their own streams: 67 x 45 x 51 box (D3Q19
+// BF16) 8 planes 31.8 / 14.0, 4 planes (chosen) 22.0 / 11.2, 2 planes 20.6 / 14.1; 32 x
+// 32 x 64 jet (D3Q27 FP32) 8: 33.9 / 11.9, 2 (chosen): 19.5 / 8.6, 1: 19.6 / 9.8; 48 x 48
+// x 96 (D3Q19 FP32) 8: 28.7 / 16.3, 4 (chosen): 23.6 / 14.5, 2: 25.7 / 17.1.  Beyond two
+// items per SM the prologues cost what the latency gains (83 x 83 x 84 box, D3Q27
+// BF16, 8: 53 / 36, 5: 45 / 41).
+inline int small_chunk(long cols, int nzf, int zchunk, int sms) {
+    double best = 1e300;
+    int arg = zchunk;
+    for (int zc = 2; zc <= zchunk; ++zc) {
+        const long items = cols * ((nzf + zc - 1) / zc);
+        if (items > 2l * sms) continue;
+        const double t = (zc + kProloguePlanes) * (items > sms ? 1.25 : 1.0);
+        if (t <= best) { // ties: the longer chunk
+            best = t;
+            arg = zc;
+        }
+    }
+    return arg;
+}
+
 // Bulk tiling: 32 x 8 columns.  Unless the caller fixes tile_z, the z chunk
 // (8..64 planes, the range the model was checked on) minimises
-// chunk_makespan; the choice is cached per lattice shape and slot count (the
-// search costs a few ms on the largest lattices).
-inline void tiling(const ssmd_params &p, const Geometry &G, int slots, int &tiles_x, int &tiles_y,
+// chunk_makespan, and where that is 8 small_chunk decides; the choice is cached
+// per lattice shape and slot count (the search costs a few ms on the largest
+// lattices).
+inline void tiling(const ssmd_params &p, const Geometry &G, int slots, int sms, int &tiles_x, int &tiles_y,
                    int &zchunk, int &nchunks) {
     tiles_x = (int)((G.nx + kTX - 1) / kTX);
     tiles_y = (int)((G.ny + kTY - 1) / kTY);
@@ -238,6 +265,7 @@ inline void tiling(const ssmd_params &p, const Geometry &G, int slots, int &tile
                     arg = zc;
                 }
             }
+            if (arg <= 8) arg = small_chunk(cols, nzf, arg, sms);
             c_cols = cols;
             c_nzf = nzf;
             c_slots = slots;
@@ -295,7 +323,7 @@ int launch_step(const ssmd_params &p, const LBMFields &fl, uint64_t step, uint32
         if constexpr (kSlabs) bulk_slots<Q, T, 3>(per_sm, sms);
     } else if (pxy) bulk_slots<Q, T, 1, true>(per_sm, sms);
     else bulk_slots<Q, T, 1>(per_sm, sms);
-    tiling(p, a.geo, per_sm * sms, a.tiles_x, a.tiles_y, a.zchunk, a.nzchunks);
+    tiling(p, a.geo, per_sm * sms, sms, a.tiles_x, a.tiles_y, a.zchunk, a.nzchunks);
     a.halo_mod = (a.geo.bcx == BC_PERIODIC && a.geo.nx < (uint32_t)(kTX + 4)) ||
                  (a.geo.bcy == BC_PERIODIC && a.geo.ny < (uint32_t)(kTY + 4)) ||
                  (a.geo.bcz == BC_PERIODIC && a.geo.nz < 6u);
