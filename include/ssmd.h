@@ -465,7 +465,13 @@ int ssmd_derived_update(const ssmd_params *p, const LBMFields *fields, uint32_t 
  *   ssmd_mlp_average: avg = decay * avg + (1 - decay) * net on the params (an
  *     exponential moving average of the weights along training; the
  *     normalisation part of avg is left as it is).
- *   ssmd_mlp_status: bit 0 set when an MMA wait timed out (the CTA aborted).
+ *   ssmd_mlp_train_step: one training step on a mini-batch, the same bits as
+ *     gathering rows rows[0 .. batch - 1] (device, int64) of features, targets and
+ *     weights (n_rows rows each), then ssmd_mlp_grad_ws, ssmd_mlp_adam and, when avg
+ *     is not NULL, ssmd_mlp_average(avg, net, decay); two kernels.  A row index
+ *     outside [0, n_rows) contributes nothing and sets bit 1 of the status.
+ *   ssmd_mlp_status: bit 0 set when an MMA wait timed out (the CTA aborted), bit 1
+ *     when a training step met a row index out of range.
  * Features (ssmd_closure_features), per cell, from rho, ux, uy, uz, phi with
  * central differences (periodic axes wrap, others clamp at the faces):
  *   phi, 4 phi (1 - phi), |grad phi|, laplacian phi, |S| = sqrt(2 S:S),
@@ -497,6 +503,10 @@ int ssmd_mlp_grad_ws(const float *net, const float *features, const float *targe
 int ssmd_mlp_adam(float *net, const float *grad, float *m, float *v, int64_t t, float lr, float beta1,
                   float beta2, float eps, ssmd_stream_t stream);
 int ssmd_mlp_average(float *avg, const float *net, float decay, ssmd_stream_t stream);
+int ssmd_mlp_train_step(float *net, const float *features, const float *targets, const float *weights,
+                        int64_t n_rows, const int64_t *rows, int64_t batch, float *grad, double *loss, float *m,
+                        float *v, int64_t t, float lr, float beta1, float beta2, float eps, float *avg, float decay,
+                        float *workspace, size_t workspace_bytes, ssmd_stream_t stream);
 int ssmd_mlp_status(uint32_t *status);
 int ssmd_closure_features(const ssmd_params *p, const LBMFields *fields, float *features, ssmd_stream_t stream);
 int ssmd_closure_filter(const ssmd_params *fine, const LBMFields *fine_fields, float *coarse, float *tau,

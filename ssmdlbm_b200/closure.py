@@ -129,21 +129,36 @@ class Network:
         gen.manual_seed(seed)
         n = feats.shape[0]
         b = min(batch, n)
-        fb = torch.empty(b, feats.shape[1], device=self.device)
-        tb = torch.empty(b, 2, device=self.device)
-        wb = torch.empty(b, 2, device=self.device)
         losses = []
+        # plain float32 rows on the network's device are read through their indices in the
+        # training kernel (ssmd_mlp_train_step); anything else is gathered first, as torch
+        # accepts or refuses it
+        direct = all(type(v) is torch.Tensor and v.dtype == torch.float32 and v.device == self.net.device
+                     and v.is_contiguous() and not v.requires_grad and tuple(v.shape) == (n, c)
+                     for v, c in ((feats, _lib.MLP_IN), (targets, 2), (weights, 2)))
+        if not direct:
+            fb = torch.empty(b, feats.shape[1], device=self.device)
+            tb = torch.empty(b, 2, device=self.device)
+            wb = torch.empty(b, 2, device=self.device)
         for k in range(steps):
             idx = torch.randint(0, n, (b,), device=self.device, generator=gen)
-            torch.index_select(feats, 0, idx, out=fb)
-            torch.index_select(targets, 0, idx, out=tb)
-            torch.index_select(weights, 0, idx, out=wb)
-            self._grad(fb, tb, wb, b, st)
-            self.t += 1
-            check(L.ssmd_mlp_adam(self.net.data_ptr(), self.grad.data_ptr(), self.m.data_ptr(), self.v.data_ptr(),
-                                  self.t, lr, 0.9, 0.999, 1e-8, st))
-            if avg is not None:
-                check(L.ssmd_mlp_average(avg.data_ptr(), self.net.data_ptr(), average, st))
+            if direct:
+                check(L.ssmd_mlp_train_step(
+                    self.net.data_ptr(), feats.data_ptr(), targets.data_ptr(), weights.data_ptr(), n, idx.data_ptr(), b,
+                    self.grad.data_ptr(), self.loss.data_ptr(), self.m.data_ptr(), self.v.data_ptr(), self.t + 1, lr, 0.9,
+                    0.999, 1e-8, avg.data_ptr() if avg is not None else None, average if avg is not None else 0.0,
+                    self.ws.data_ptr(), self.ws.numel() * 4, st))
+                self.t += 1
+            else:
+                torch.index_select(feats, 0, idx, out=fb)
+                torch.index_select(targets, 0, idx, out=tb)
+                torch.index_select(weights, 0, idx, out=wb)
+                self._grad(fb, tb, wb, b, st)
+                self.t += 1
+                check(L.ssmd_mlp_adam(self.net.data_ptr(), self.grad.data_ptr(), self.m.data_ptr(), self.v.data_ptr(),
+                                      self.t, lr, 0.9, 0.999, 1e-8, st))
+                if avg is not None:
+                    check(L.ssmd_mlp_average(avg.data_ptr(), self.net.data_ptr(), average, st))
             if report_every and (k % report_every == 0 or k == steps - 1):
                 losses.append((k, float(self.loss.item())))
         if avg is not None:

@@ -55,6 +55,7 @@ namespace {
 
 constexpr int kIn = SSMD_MLP_IN, kK1 = 16, kH = SSMD_MLP_HIDDEN, kOut = SSMD_MLP_OUT, kN3 = 16;
 constexpr int kRows = 128, kThreadsMlp = 128;
+constexpr int kTrainGroups = 4, kThreadsTrain = kTrainGroups * kRows; // training: 16 columns of a row per thread
 constexpr int oW1 = 0, oB1 = oW1 + kH * kK1, oW2 = oB1 + kH, oB2 = oW2 + kH * kH, oW3 = oB2 + kH,
               oB3 = oW3 + kOut * kH, kParams = oB3 + kOut;
 constexpr int oMean = kParams, oInvStd = oMean + kIn, oScale = oInvStd + kIn, oOffset = oScale + kOut,
@@ -115,6 +116,8 @@ struct MlpArgs {
     const float *feat;   // kFwd, kTrain: n x 12 features
     const float *target; // kTrain
     const float *weight; // kTrain (may be null)
+    const int64_t *rows; // kTrain: row i of the batch is row rows[i] of feat, target, weight (null: row i)
+    int64_t n_rows;      // kTrain: rows of feat, target, weight
     int64_t n;
     float *out;          // kFwd: n x 2
     float *grad;         // kTrain: atomics into grad, or null with partials
@@ -177,8 +180,8 @@ __device__ __forceinline__ void st8(unsigned char *tile, int r, int k0, int K, c
 // power of two), into a bf16 tile of rows_pad rows (extra rows zero);
 // transpose: element (r, k) = src[k * rows + r].
 __device__ void load_weights(unsigned char *tile, const float *src, int rows, int rows_pad, int K, bool transpose,
-                             int tid, float scale = 1.0f) {
-    for (int e = tid; e < rows_pad * K; e += kThreadsMlp) {
+                             int tid, int threads, float scale = 1.0f) {
+    for (int e = tid; e < rows_pad * K; e += threads) {
         const int r = e / K, k = e % K;
         float v = 0.f;
         if (r < rows) v = transpose ? src[k * rows + r] : src[r * K + k];
@@ -205,14 +208,27 @@ __device__ __forceinline__ uint16_t bf16_bits(float v) {
     return *reinterpret_cast<const uint16_t *>(&h);
 }
 
-// Bias + GELU epilogue of a 64-column accumulator into a [128 x 64] bf16 tile
-// (TWICE: 2 gelu, for a next layer staged with halved weights; TRANS: the
-// same bf16 values also into column r, rows trow0 .. trow0 + 63, of a
-// weight-gradient operand tile).  The TMEM load of columns 16 (c + 1) ..
-// 16 c + 31 is in flight while columns 16 c .. 16 c + 15 are processed.
-template <bool TWICE = false, bool TRANS = false>
-__device__ __forceinline__ void hidden_epilogue(uint32_t taddr, const float *bias, unsigned char *tile, int r,
-                                                unsigned char *ttile = nullptr, int trow0 = 0) {
+// Bias + GELU of 16 accumulator columns v (columns c0 .. c0 + 15 of the layer)
+// into row r of a [128 x 64] bf16 tile (TWICE: 2 gelu, for a next layer staged
+// with halved weights); pk returns the bf16 pairs.
+template <bool TWICE>
+__device__ __forceinline__ void gelu16(const float (&v)[16], const float *bias, int c0, unsigned char *tile, int r,
+                                       uint32_t (&pk)[8]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 b = *reinterpret_cast<const float4 *>(bias + c0 + 4 * i);
+        const float2 g0 = gelu2<TWICE>(__fadd2_rn(make_float2(v[4 * i], v[4 * i + 1]), make_float2(b.x, b.y)));
+        const float2 g1 = gelu2<TWICE>(__fadd2_rn(make_float2(v[4 * i + 2], v[4 * i + 3]), make_float2(b.z, b.w)));
+        pk[2 * i] = pack2(g0.x, g0.y);
+        pk[2 * i + 1] = pack2(g1.x, g1.y);
+    }
+    *reinterpret_cast<uint4 *>(tile + umma::kmajor_offset(r, c0, kH)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+    *reinterpret_cast<uint4 *>(tile + umma::kmajor_offset(r, c0 + 8, kH)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+}
+
+// Inference epilogue of a 64-column accumulator: the TMEM load of columns
+// 16 (c + 1) .. 16 c + 31 is in flight while columns 16 c .. 16 c + 15 are processed.
+__device__ __forceinline__ void hidden_epilogue(uint32_t taddr, const float *bias, unsigned char *tile, int r) {
     uint32_t nxt[16];
     umma::tmem_ld16_issue(taddr, nxt);
 #pragma unroll
@@ -223,24 +239,22 @@ __device__ __forceinline__ void hidden_epilogue(uint32_t taddr, const float *bia
         for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(nxt[i]);
         if (c < 3) umma::tmem_ld16_issue(taddr + 16 * (c + 1), nxt);
         uint32_t pk[8];
+        gelu16<true>(v, bias, 16 * c, tile, r, pk);
+    }
+}
+
+// Training epilogue of columns 16 grp .. 16 grp + 15: the same bf16 values also
+// into column r, rows trow0 + 16 grp .., of a weight-gradient operand tile.
+__device__ __forceinline__ void hidden_epilogue16(uint32_t taddr, const float *bias, unsigned char *tile, int r, int grp,
+                                                  unsigned char *ttile, int trow0) {
+    float v[16];
+    umma::tmem_ld16(taddr + 16 * grp, v);
+    uint32_t pk[8];
+    gelu16<false>(v, bias, 16 * grp, tile, r, pk);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float4 b = *reinterpret_cast<const float4 *>(bias + 16 * c + 4 * i);
-            const float2 g0 = gelu2<TWICE>(__fadd2_rn(make_float2(v[4 * i], v[4 * i + 1]), make_float2(b.x, b.y)));
-            const float2 g1 = gelu2<TWICE>(__fadd2_rn(make_float2(v[4 * i + 2], v[4 * i + 3]), make_float2(b.z, b.w)));
-            pk[2 * i] = pack2(g0.x, g0.y);
-            pk[2 * i + 1] = pack2(g1.x, g1.y);
-        }
-        if constexpr (TRANS) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                st_g(ttile, trow0 + 16 * c + 2 * i, r, (uint16_t)(pk[i] & 0xFFFFu));
-                st_g(ttile, trow0 + 16 * c + 2 * i + 1, r, (uint16_t)(pk[i] >> 16));
-            }
-        }
-        *reinterpret_cast<uint4 *>(tile + umma::kmajor_offset(r, 16 * c, kH)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-        *reinterpret_cast<uint4 *>(tile + umma::kmajor_offset(r, 16 * c + 8, kH)) =
-            make_uint4(pk[4], pk[5], pk[6], pk[7]);
+    for (int i = 0; i < 8; ++i) {
+        st_g(ttile, trow0 + 16 * grp + 2 * i, r, (uint16_t)(pk[i] & 0xFFFFu));
+        st_g(ttile, trow0 + 16 * grp + 2 * i + 1, r, (uint16_t)(pk[i] >> 16));
     }
 }
 
@@ -276,8 +290,8 @@ __device__ __forceinline__ void load_row(const MlpArgs &a, const float *norm, in
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kThreadsMlp, MODE == kTrain ? 1 : 7) mlp_kernel(const MlpArgs a) {
-    constexpr bool TRAIN = MODE == kTrain;
+__global__ void __launch_bounds__(kThreadsMlp, 7) mlp_kernel(const MlpArgs a) {
+    static_assert(MODE == kFwd || MODE == kRefresh, "training has its own kernel");
     using L = Layout<MODE>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + (L::align - 1)) &
@@ -288,7 +302,6 @@ __global__ void __launch_bounds__(kThreadsMlp, MODE == kTrain ? 1 : 7) mlp_kerne
     float *b1 = reinterpret_cast<float *>(sm + L::b1);
     float *b2 = reinterpret_cast<float *>(sm + L::b2);
     float *b3 = reinterpret_cast<float *>(sm + L::b3);
-    float *w3f = reinterpret_cast<float *>(sm + L::w3f);
     float *norm = reinterpret_cast<float *>(sm + L::norm);
     uint64_t *bar = reinterpret_cast<uint64_t *>(sm + L::bar);
     uint32_t *slot = reinterpret_cast<uint32_t *>(sm + L::slot);
@@ -301,39 +314,22 @@ __global__ void __launch_bounds__(kThreadsMlp, MODE == kTrain ? 1 : 7) mlp_kerne
         *abort_flag = 0u;
         fence_barrier_init();
     }
-    load_weights(sm + L::sW1, net + oW1, kH, kH, kK1, false, tid);
-    // inference feeds W2 and W3 with 2 gelu(z): halved weights, the same products
-    load_weights(sm + L::sW2, net + oW2, kH, kH, kH, false, tid, TRAIN ? 1.0f : 0.5f);
-    load_weights(sm + L::sW3, net + oW3, kOut, kN3, kH, false, tid, TRAIN ? 1.0f : 0.5f);
-    if constexpr (TRAIN) load_weights(sm + sW2T, net + oW2, kH, kH, kH, true, tid); // (i, o) = W2[o][i]
+    // W2 and W3 are fed with 2 gelu(z): halved weights, the same products
+    load_weights(sm + L::sW1, net + oW1, kH, kH, kK1, false, tid, kThreadsMlp);
+    load_weights(sm + L::sW2, net + oW2, kH, kH, kH, false, tid, kThreadsMlp, 0.5f);
+    load_weights(sm + L::sW3, net + oW3, kOut, kN3, kH, false, tid, kThreadsMlp, 0.5f);
     for (int e = tid; e < kH; e += kThreadsMlp) {
         b1[e] = net[oB1 + e];
         b2[e] = net[oB2 + e];
     }
-    if constexpr (TRAIN)
-        for (int e = tid; e < kOut * kH; e += kThreadsMlp) w3f[e] = net[oW3 + e];
     if (tid < kOut) b3[tid] = net[oB3 + tid];
     if (tid < kNet - kParams) norm[tid] = net[kParams + tid];
-    if constexpr (TRAIN) {
-        // the rows of the gradient operands that no tile writes: GA2 row 12
-        // all ones (its products are the column sums, the bias gradients),
-        // rows 13-15 and GB rows 130-143 zero
-        const uint16_t one = bf16_bits(1.0f);
-        st_g(sm + sGA2, 12, tid, one);
-        for (int m = 13; m < 16; ++m) st_g(sm + sGA2, m, tid, 0);
-        for (int m = 2 * kH + kOut; m < kGB; ++m) st_g(sm + sGB, m, tid, 0);
-    }
     __syncthreads();
 
     const int r = tid;
     const uint32_t sbase = smem_addr(sm);
     uint32_t phase = 0;
     bool ok = true;
-    // training: the weight-gradient MMAs of a tile run while the next tile's
-    // features load; gpend says they are in flight (waited for before the
-    // next tile writes their operands, and after the last tile)
-    bool gpend = false, gfirst = true;
-    float lsum = 0.f;
     const int64_t tiles = (n + kRows - 1) / kRows;
     uint32_t tmem = 0, lane_base = 0;
 
@@ -346,16 +342,6 @@ __global__ void __launch_bounds__(kThreadsMlp, MODE == kTrain ? 1 : 7) mlp_kerne
             load_row<MODE>(a, norm, row, valid, x, nu_phi);
             st8(sm + L::sX, r, 0, kK1, x);
             st8(sm + L::sX, r, 8, kK1, x + 8);
-            if constexpr (TRAIN) {
-                if (gpend) { // the previous tile's gradient MMAs read GA2, GA1, GB
-                    ok = wait_mma(bar, phase, abort_flag);
-                    phase ^= 1u;
-                    gpend = false;
-                    if (!ok) break;
-                }
-#pragma unroll
-                for (int k = 0; k < kIn; ++k) st_g(sm + sGA2, k, r, bf16_bits(x[k])); // X^T
-            }
         }
         fence_proxy_async(); // generic-proxy smem writes -> visible to the tensor core
         umma::fence_before_sync();
@@ -373,7 +359,7 @@ __global__ void __launch_bounds__(kThreadsMlp, MODE == kTrain ? 1 : 7) mlp_kerne
         ok = wait_mma(bar, phase, abort_flag);
         phase ^= 1u;
         if (!ok) break;
-        hidden_epilogue<!TRAIN, TRAIN>(lane_base + cZ1, b1, sm + L::sH1, r, sm + sGA1, 0); // (H1^T)
+        hidden_epilogue(lane_base + cZ1, b1, sm + L::sH1, r);
         fence_proxy_async();
         umma::fence_before_sync();
         __syncthreads();
@@ -390,7 +376,7 @@ __global__ void __launch_bounds__(kThreadsMlp, MODE == kTrain ? 1 : 7) mlp_kerne
         ok = wait_mma(bar, phase, abort_flag);
         phase ^= 1u;
         if (!ok) break;
-        hidden_epilogue<!TRAIN, TRAIN>(lane_base + col_z2<MODE>(), b2, sm + L::sH2, r, sm + sGA1, kH); // (H2^T)
+        hidden_epilogue(lane_base + col_z2<MODE>(), b2, sm + L::sH2, r);
         fence_proxy_async();
         umma::fence_before_sync();
         __syncthreads();
@@ -419,7 +405,7 @@ __global__ void __launch_bounds__(kThreadsMlp, MODE == kTrain ? 1 : 7) mlp_kerne
                 *reinterpret_cast<float2 *>(a.out + row * kOut) =
                     make_float2(fmaf(norm[2 * kIn + 0], rr[0], norm[2 * kIn + 2]),
                                 fmaf(norm[2 * kIn + 1], rr[1], norm[2 * kIn + 3]));
-        } else if constexpr (MODE == kRefresh) {
+        } else {
             // the closure's bounds (ssmd_closure_apply): nu_t >= max(-nu(phi)/2, -nut_max)
             if (valid) {
                 const float p0 = fmaf(norm[2 * kIn + 0], rr[0], norm[2 * kIn + 2]);
@@ -427,145 +413,6 @@ __global__ void __launch_bounds__(kThreadsMlp, MODE == kTrain ? 1 : 7) mlp_kerne
                 const float lo = fmaxf(-0.5f * nu_phi, -a.nut_max);
                 a.nut[row] = fminf(fmaxf(p0, lo), a.nut_max);
                 a.cs[row] = fminf(fmaxf(p1, 0.25f), 4.0f);
-            }
-        } else {
-            // ---- loss and dL/dr
-            float d0 = 0.f, d1 = 0.f;
-            if (valid) {
-                const float inv_n = 1.0f / (float)n;
-                const float t0 = (a.target[row * kOut + 0] - norm[2 * kIn + 2]) / norm[2 * kIn + 0];
-                const float t1 = (a.target[row * kOut + 1] - norm[2 * kIn + 3]) / norm[2 * kIn + 1];
-                const float w0 = a.weight ? a.weight[row * kOut + 0] : 1.0f;
-                const float w1 = a.weight ? a.weight[row * kOut + 1] : 1.0f;
-                const float e0 = rr[0] - t0, e1 = rr[1] - t1;
-                lsum += w0 * e0 * e0 + w1 * e1 * e1;
-                d0 = 2.0f * w0 * e0 * inv_n;
-                d1 = 2.0f * w1 * e1 * inv_n;
-            }
-            st_g(sm + sGB, 2 * kH + 0, r, bf16_bits(d0)); // dR^T
-            st_g(sm + sGB, 2 * kH + 1, r, bf16_bits(d1));
-            // ---- dZ2 = (dR W3) * gelu'(z2 + b2)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                float v[16];
-                umma::tmem_ld16(lane_base + col_z2<MODE>() + 16 * c, v);
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int j = 16 * c + i;
-                    const float dh = fmaf(d0, w3f[j], d1 * w3f[kH + j]);
-                    v[i] = dh * gelu_grad(v[i] + b2[j]);
-                    st_g(sm + sGB, kH + j, r, bf16_bits(v[i])); // dZ2^T
-                }
-                st8(sm + sDZ2, r, 16 * c, kH, v);
-                st8(sm + sDZ2, r, 16 * c + 8, kH, v + 8);
-            }
-            fence_proxy_async();
-            umma::fence_before_sync();
-            __syncthreads();
-            // ---- dH1 = dZ2 W2 (B = W2^T, K-major)
-            if (tid == 0) {
-                umma::fence_after_sync();
-                for (int ks = 0; ks < kH / 16; ++ks)
-                    umma::mma_bf16(tmem + cDH1, umma::smem_desc(sbase + sDZ2 + 256 * ks, 128, 1024),
-                                   umma::smem_desc(sbase + sW2T + 256 * ks, 128, 1024), umma::idesc_bf16(128, kH),
-                                   ks > 0);
-                umma::commit(bar);
-            }
-            ok = wait_mma(bar, phase, abort_flag);
-            phase ^= 1u;
-            if (!ok) break;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                float dh[16], z[16];
-                umma::tmem_ld16(lane_base + cDH1 + 16 * c, dh);
-                umma::tmem_ld16(lane_base + cZ1 + 16 * c, z);
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    st_g(sm + sGB, 16 * c + i, r, bf16_bits(dh[i] * gelu_grad(z[i] + b1[16 * c + i]))); // dZ1^T
-            }
-            fence_proxy_async();
-            umma::fence_before_sync();
-            __syncthreads();
-            // ---- weight and bias gradients of this tile, summed over its 128
-            // rows (the MMAs' K) into the CTA's accumulators G1 and G2:
-            //   G1 [128 x 80]  += GA1 GB[64..143]^T: rows 0-63 dW2^T, rows 64-127 cols 64-65 dW3^T
-            //   G2 [128 x 144] += GA2 GB^T: rows 0-11 cols 0-63 dW1^T; row 12: db1, db2, db3
-            if (tid == 0) {
-                umma::fence_after_sync();
-                for (int ks = 0; ks < kGK / 16; ++ks)
-                    umma::mma_bf16(tmem + cG1, umma::smem_desc(sbase + sGA1 + 256 * ks, 128, 2048),
-                                   umma::smem_desc(sbase + sGB + (kH / 8) * 2048 + 256 * ks, 128, 2048),
-                                   umma::idesc_bf16(128, kGB - kH), !gfirst || ks > 0);
-                for (int ks = 0; ks < kGK / 16; ++ks)
-                    umma::mma_bf16(tmem + cG2, umma::smem_desc(sbase + sGA2 + 256 * ks, 128, 2048),
-                                   umma::smem_desc(sbase + sGB + 256 * ks, 128, 2048), umma::idesc_bf16(128, kGB),
-                                   !gfirst || ks > 0);
-                umma::commit(bar);
-            }
-            gpend = true;
-            gfirst = false;
-        }
-    }
-    if constexpr (TRAIN) {
-        if (ok && gpend) {
-            ok = wait_mma(bar, phase, abort_flag);
-            phase ^= 1u;
-        }
-    }
-
-    if constexpr (TRAIN) {
-        if (ok) {
-            // atomics into grad, or this CTA's row of the deterministic workspace
-            float *dst = a.partials ? a.partials + (size_t)blockIdx.x * (kParams + 1) : a.grad;
-            auto put = [&](int k, float v) {
-                if (a.partials) dst[k] = v;
-                else atomicAdd(&dst[k], v);
-            };
-            // thread m reads row m of the accumulators (warp w holds lanes 32 w ..)
-            const int m = tid;
-            if (!gfirst) {
-                const uint32_t lb = *slot + ((uint32_t)(warp * 32) << 16);
-                float v[16];
-                if (m < kH) { // dW2[o][m] = G1[m][o]
-#pragma unroll
-                    for (int c = 0; c < kH / 16; ++c) {
-                        umma::tmem_ld16(lb + cG1 + 16 * c, v);
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) put(oW2 + (16 * c + i) * kH + m, v[i]);
-                    }
-                } else { // dW3[k][m - 64] = G1[m][64 + k]
-                    umma::tmem_ld16(lb + cG1 + kH, v);
-                    put(oW3 + 0 * kH + (m - kH), v[0]);
-                    put(oW3 + 1 * kH + (m - kH), v[1]);
-                }
-                if (warp == 0) { // warp-collective loads: lanes 0-11 dW1, lane 12 the biases
-                    for (int c = 0; c < kGB / 16; ++c) {
-                        umma::tmem_ld16(lb + cG2 + 16 * c, v);
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) {
-                            const int col = 16 * c + i;
-                            if (col < kH && m < kK1) put(oW1 + col * kK1 + m, m < kIn ? v[i] : 0.f); // dW1[o][m]
-                            if (m == kIn) {
-                                if (col < kH) put(oB1 + col, v[i]);
-                                else if (col < 2 * kH) put(oB2 + col - kH, v[i]);
-                                else if (col < 2 * kH + kOut) put(oB3 + col - 2 * kH, v[i]);
-                            }
-                        }
-                    }
-                }
-            } else { // a CTA without tiles adds zeros
-                for (int e = tid; e < kParams; e += kThreadsMlp) put(e, 0.f);
-            }
-            float l = lsum;
-            for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
-            if (a.partials) {
-                float *wl = reinterpret_cast<float *>(sm + sDY); // per-warp losses, summed in warp order
-                __syncthreads();
-                if ((tid & 31) == 0) wl[warp] = l;
-                __syncthreads();
-                if (tid == 0) dst[kParams] = ((wl[0] + wl[1]) + wl[2]) + wl[3];
-            } else if ((tid & 31) == 0) {
-                atomicAdd(a.loss, (double)l / (double)n);
             }
         }
     }
@@ -577,20 +424,381 @@ __global__ void __launch_bounds__(kThreadsMlp, MODE == kTrain ? 1 : 7) mlp_kerne
     if (warp == 0) umma::tmem_dealloc(*slot, tmem_cols<MODE>());
 }
 
-// Deterministic reduction of the per-CTA gradient rows: thread k sums column
-// k over the CTAs in CTA order (FP32, like the atomic path); the loss column
-// in FP64.
-__global__ void grad_sum_kernel(const float *__restrict__ partials, int ctas, int64_t n, float *__restrict__ grad,
-                                double *__restrict__ loss) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// What a training thread holds of one row before its tile begins: features
+// 4 grp .. 4 grp + 3 (groups 0-2), targets and weights.
+struct TrainRow {
+    float4 f;
+    float t0, t1, w0, w1;
+    bool valid;
+};
+
+// Training: 512 threads per CTA, one CTA per SM (512 TMEM columns).  Thread (grp,
+// r) handles row r and, of every 64-column layer, columns 16 grp .. 16 grp + 15.  The
+// kernel is a chain of MMA round trips and epilogues per tile; with one thread
+// per row (4 warps per SM, one per scheduler) the epilogues' ~5000 instructions
+// ran at the latency of one warp: 15 us a tile, 62 us for 65 536 rows; with four
+// threads per row LLL.  The rows of a mini-batch are read through their
+// indices (a.rows), the next tile's while this one's layers run: gathering them first took
+// three launches and 50 us of the 128 us step.  Every value and every sum is in
+// the order of one thread per row: the same bits.
+__global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpArgs a) {
+    using L = Layout<kTrain>;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + (L::align - 1)) &
+                                                          ~(uintptr_t)(L::align - 1));
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int r = tid & (kRows - 1), grp = tid / kRows;
+    const float *net = a.net;
+    const int64_t n = a.n;
+    float *b1 = reinterpret_cast<float *>(sm + L::b1);
+    float *b2 = reinterpret_cast<float *>(sm + L::b2);
+    float *b3 = reinterpret_cast<float *>(sm + L::b3);
+    float *w3f = reinterpret_cast<float *>(sm + L::w3f);
+    float *norm = reinterpret_cast<float *>(sm + L::norm);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + L::bar);
+    uint32_t *slot = reinterpret_cast<uint32_t *>(sm + L::slot);
+    volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(sm + L::abort);
+    const int64_t tiles = (n + kRows - 1) / kRows;
+
+    // the source row of this thread's row of a tile; -1: none
+    auto source = [&](int64_t tile) -> int64_t {
+        const int64_t row = tile * kRows + r;
+        if (row >= n) return -1;
+        if (!a.rows) return row;
+        const int64_t s = __ldg(a.rows + row);
+        if (s >= 0 && s < a.n_rows) return s;
+        if (grp == 0) atomicOr(&g_mlp_status, 2u);
+        return -1;
+    };
+    const bool aligned = (reinterpret_cast<uintptr_t>(a.feat) & 15u) == 0; // 48-byte rows: 16-byte aligned
+    auto fetch = [&](int64_t s) -> TrainRow {
+        TrainRow d;
+        d.f = make_float4(0.f, 0.f, 0.f, 0.f);
+        d.t0 = d.t1 = d.w0 = d.w1 = 0.f;
+        d.valid = s >= 0;
+        if (!d.valid) return d;
+        if (grp < kIn / 4) {
+            const float *p = a.feat + s * kIn + 4 * grp;
+            if (aligned) d.f = __ldg(reinterpret_cast<const float4 *>(p));
+            else d.f = make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+        }
+        d.t0 = a.target[s * kOut + 0];
+        d.t1 = a.target[s * kOut + 1];
+        d.w0 = a.weight ? a.weight[s * kOut + 0] : 1.0f;
+        d.w1 = a.weight ? a.weight[s * kOut + 1] : 1.0f;
+        return d;
+    };
+    TrainRow cur = fetch((int64_t)blockIdx.x < tiles ? source(blockIdx.x) : -1);
+
+    // ---- set-up: TMEM, barrier, weights
+    if (warp == 0) umma::tmem_alloc(slot, tmem_cols<kTrain>());
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        *abort_flag = 0u;
+        fence_barrier_init();
+    }
+    load_weights(sm + L::sW1, net + oW1, kH, kH, kK1, false, tid, kThreadsTrain);
+    load_weights(sm + L::sW2, net + oW2, kH, kH, kH, false, tid, kThreadsTrain);
+    load_weights(sm + L::sW3, net + oW3, kOut, kN3, kH, false, tid, kThreadsTrain);
+    load_weights(sm + sW2T, net + oW2, kH, kH, kH, true, tid, kThreadsTrain); // (i, o) = W2[o][i]
+    if (tid < kH) {
+        b1[tid] = net[oB1 + tid];
+        b2[tid] = net[oB2 + tid];
+    }
+    if (tid < kOut * kH) w3f[tid] = net[oW3 + tid];
+    if (tid < kOut) b3[tid] = net[oB3 + tid];
+    if (tid < kNet - kParams) norm[tid] = net[kParams + tid];
+    if (grp == 0) {
+        // the rows of the gradient operands that no tile writes: GA2 row 12
+        // all ones (its products are the column sums, the bias gradients),
+        // rows 13-15 and GB rows 130-143 zero
+        const uint16_t one = bf16_bits(1.0f);
+        st_g(sm + sGA2, 12, r, one);
+        for (int m = 13; m < 16; ++m) st_g(sm + sGA2, m, r, 0);
+        for (int m = 2 * kH + kOut; m < kGB; ++m) st_g(sm + sGB, m, r, 0);
+    }
+    __syncthreads();
+
+    const uint32_t sbase = smem_addr(sm);
+    uint32_t phase = 0;
+    bool ok = true;
+    // the weight-gradient MMAs of a tile run while the next tile begins; gpend
+    // says they are in flight (waited for before the next tile writes their
+    // operands, and after the last tile)
+    bool gpend = false, gfirst = true;
+    float lsum = 0.f;
+    const uint32_t tmem = *slot;
+    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+
+    for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        const int64_t next = tile + gridDim.x;
+        const int64_t nsrc = next < tiles ? source(next) : -1;
+        {
+            // group 3 writes the zero padding of X (columns 12-15)
+            float x[4];
+            const float f[4] = {cur.f.x, cur.f.y, cur.f.z, cur.f.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                x[i] = cur.valid && grp < kIn / 4 ? (f[i] - norm[4 * grp + i]) * norm[kIn + 4 * grp + i] : 0.f;
+            *reinterpret_cast<uint2 *>(sm + L::sX + umma::kmajor_offset(r, 4 * grp, kK1)) =
+                make_uint2(pack2(x[0], x[1]), pack2(x[2], x[3]));
+            if (gpend) { // the previous tile's gradient MMAs read GA2, GA1, GB
+                ok = wait_mma(bar, phase, abort_flag);
+                phase ^= 1u;
+                gpend = false;
+                if (!ok) break;
+            }
+            if (grp < kIn / 4) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) st_g(sm + sGA2, 4 * grp + i, r, bf16_bits(x[i])); // X^T
+            }
+        }
+        fence_proxy_async(); // generic-proxy smem writes -> visible to the tensor core
+        umma::fence_before_sync();
+        __syncthreads(); // also: every TMEM read and MMA of the previous tile is complete
+
+        // ---- layer 1
+        if (tid == 0) {
+            umma::fence_after_sync();
+            umma::mma_bf16(tmem + cZ1, umma::smem_desc(sbase + L::sX, 128, 256),
+                           umma::smem_desc(sbase + L::sW1, 128, 256), umma::idesc_bf16(128, kH), false);
+            umma::commit(bar);
+        }
+        const TrainRow nxt = fetch(nsrc);
+        ok = wait_mma(bar, phase, abort_flag);
+        phase ^= 1u;
+        if (!ok) break;
+        hidden_epilogue16(lane_base + cZ1, b1, sm + L::sH1, r, grp, sm + sGA1, 0); // (H1^T)
+        fence_proxy_async();
+        umma::fence_before_sync();
+        __syncthreads();
+
+        // ---- layer 2
+        if (tid == 0) {
+            umma::fence_after_sync();
+            for (int ks = 0; ks < kH / 16; ++ks)
+                umma::mma_bf16(tmem + col_z2<kTrain>(), umma::smem_desc(sbase + L::sH1 + 256 * ks, 128, 1024),
+                               umma::smem_desc(sbase + L::sW2 + 256 * ks, 128, 1024), umma::idesc_bf16(128, kH),
+                               ks > 0);
+            umma::commit(bar);
+        }
+        ok = wait_mma(bar, phase, abort_flag);
+        phase ^= 1u;
+        if (!ok) break;
+        hidden_epilogue16(lane_base + col_z2<kTrain>(), b2, sm + L::sH2, r, grp, sm + sGA1, kH); // (H2^T)
+        fence_proxy_async();
+        umma::fence_before_sync();
+        __syncthreads();
+
+        // ---- layer 3 (N padded to 16; rows 2..15 of W3 are zero)
+        if (tid == 0) {
+            umma::fence_after_sync();
+            for (int ks = 0; ks < kH / 16; ++ks)
+                umma::mma_bf16(tmem + col_r<kTrain>(), umma::smem_desc(sbase + L::sH2 + 256 * ks, 128, 1024),
+                               umma::smem_desc(sbase + L::sW3 + 256 * ks, 128, 1024), umma::idesc_bf16(128, kN3),
+                               ks > 0);
+            umma::commit(bar);
+        }
+        ok = wait_mma(bar, phase, abort_flag);
+        phase ^= 1u;
+        if (!ok) break;
+        float rr[kOut];
+        {
+            float v[2];
+            umma::tmem_ld2(lane_base + col_r<kTrain>(), v);
+            rr[0] = v[0] + b3[0];
+            rr[1] = v[1] + b3[1];
+        }
+        // ---- loss and dL/dr (each of a row's threads; group 0 keeps the sum)
+        float d0 = 0.f, d1 = 0.f;
+        if (cur.valid) {
+            const float inv_n = 1.0f / (float)n;
+            const float t0 = (cur.t0 - norm[2 * kIn + 2]) / norm[2 * kIn + 0];
+            const float t1 = (cur.t1 - norm[2 * kIn + 3]) / norm[2 * kIn + 1];
+            const float e0 = rr[0] - t0, e1 = rr[1] - t1;
+            lsum += cur.w0 * e0 * e0 + cur.w1 * e1 * e1;
+            d0 = 2.0f * cur.w0 * e0 * inv_n;
+            d1 = 2.0f * cur.w1 * e1 * inv_n;
+        }
+        if (grp == 0) {
+            st_g(sm + sGB, 2 * kH + 0, r, bf16_bits(d0)); // dR^T
+            st_g(sm + sGB, 2 * kH + 1, r, bf16_bits(d1));
+        }
+        // ---- dZ2 = (dR W3) * gelu'(z2 + b2)
+        {
+            float v[16];
+            umma::tmem_ld16(lane_base + col_z2<kTrain>() + 16 * grp, v);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int j = 16 * grp + i;
+                const float dh = fmaf(d0, w3f[j], d1 * w3f[kH + j]);
+                v[i] = dh * gelu_grad(v[i] + b2[j]);
+                st_g(sm + sGB, kH + j, r, bf16_bits(v[i])); // dZ2^T
+            }
+            st8(sm + sDZ2, r, 16 * grp, kH, v);
+            st8(sm + sDZ2, r, 16 * grp + 8, kH, v + 8);
+        }
+        fence_proxy_async();
+        umma::fence_before_sync();
+        __syncthreads();
+        // ---- dH1 = dZ2 W2 (B = W2^T, K-major)
+        if (tid == 0) {
+            umma::fence_after_sync();
+            for (int ks = 0; ks < kH / 16; ++ks)
+                umma::mma_bf16(tmem + cDH1, umma::smem_desc(sbase + sDZ2 + 256 * ks, 128, 1024),
+                               umma::smem_desc(sbase + sW2T + 256 * ks, 128, 1024), umma::idesc_bf16(128, kH),
+                               ks > 0);
+            umma::commit(bar);
+        }
+        ok = wait_mma(bar, phase, abort_flag);
+        phase ^= 1u;
+        if (!ok) break;
+        {
+            float dh[16], z[16];
+            umma::tmem_ld16(lane_base + cDH1 + 16 * grp, dh);
+            umma::tmem_ld16(lane_base + cZ1 + 16 * grp, z);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int j = 16 * grp + i;
+                st_g(sm + sGB, j, r, bf16_bits(dh[i] * gelu_grad(z[i] + b1[j]))); // dZ1^T
+            }
+        }
+        fence_proxy_async();
+        umma::fence_before_sync();
+        __syncthreads();
+        // ---- weight and bias gradients of this tile, summed over its 128
+        // rows (the MMAs' K) into the CTA's accumulators G1 and G2:
+        //   G1 [128 x 80]  += GA1 GB[64..143]^T: rows 0-63 dW2^T, rows 64-127 cols 64-65 dW3^T
+        //   G2 [128 x 144] += GA2 GB^T: rows 0-11 cols 0-63 dW1^T; row 12: db1, db2, db3
+        if (tid == 0) {
+            umma::fence_after_sync();
+            for (int ks = 0; ks < kGK / 16; ++ks)
+                umma::mma_bf16(tmem + cG1, umma::smem_desc(sbase + sGA1 + 256 * ks, 128, 2048),
+                               umma::smem_desc(sbase + sGB + (kH / 8) * 2048 + 256 * ks, 128, 2048),
+                               umma::idesc_bf16(128, kGB - kH), !gfirst || ks > 0);
+            for (int ks = 0; ks < kGK / 16; ++ks)
+                umma::mma_bf16(tmem + cG2, umma::smem_desc(sbase + sGA2 + 256 * ks, 128, 2048),
+                               umma::smem_desc(sbase + sGB + 256 * ks, 128, 2048), umma::idesc_bf16(128, kGB),
+                               !gfirst || ks > 0);
+            umma::commit(bar);
+        }
+        gpend = true;
+        gfirst = false;
+        cur = nxt;
+    }
+    if (ok && gpend) {
+        ok = wait_mma(bar, phase, abort_flag);
+        phase ^= 1u;
+    }
+
+    if (ok) {
+        // atomics into grad, or this CTA's row of the deterministic workspace
+        float *dst = a.partials ? a.partials + (size_t)blockIdx.x * (kParams + 1) : a.grad;
+        auto put = [&](int k, float v) {
+            if (a.partials) dst[k] = v;
+            else atomicAdd(&dst[k], v);
+        };
+        // the thread of row m reads row m of the accumulators, group g columns
+        // 16 g .. 16 g + 15 of G1 and every fourth 16 of G2
+        const int m = r;
+        if (!gfirst) {
+            float v[16];
+            if (m < kH) { // dW2[o][m] = G1[m][o]
+                umma::tmem_ld16(lane_base + cG1 + 16 * grp, v);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) put(oW2 + (16 * grp + i) * kH + m, v[i]);
+            } else if (grp == 0) { // dW3[k][m - 64] = G1[m][64 + k]
+                umma::tmem_ld16(lane_base + cG1 + kH, v);
+                put(oW3 + 0 * kH + (m - kH), v[0]);
+                put(oW3 + 1 * kH + (m - kH), v[1]);
+            }
+            if ((warp & 3) == 0) { // warp-collective loads: lanes 0-11 dW1, lane 12 the biases
+                for (int c = grp; c < kGB / 16; c += kTrainGroups) {
+                    umma::tmem_ld16(lane_base + cG2 + 16 * c, v);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const int col = 16 * c + i;
+                        if (col < kH && m < kK1) put(oW1 + col * kK1 + m, m < kIn ? v[i] : 0.f); // dW1[o][m]
+                        if (m == kIn) {
+                            if (col < kH) put(oB1 + col, v[i]);
+                            else if (col < 2 * kH) put(oB2 + col - kH, v[i]);
+                            else if (col < 2 * kH + kOut) put(oB3 + col - 2 * kH, v[i]);
+                        }
+                    }
+                }
+            }
+        } else { // a CTA without tiles adds zeros
+            for (int e = tid; e < kParams; e += kThreadsTrain) put(e, 0.f);
+        }
+        float l = lsum;
+        for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+        if (a.partials) {
+            float *wl = reinterpret_cast<float *>(sm + sDY); // group 0's per-warp losses, summed in warp order
+            __syncthreads();
+            if ((tid & 31) == 0 && grp == 0) wl[warp] = l;
+            __syncthreads();
+            if (tid == 0) dst[kParams] = ((wl[0] + wl[1]) + wl[2]) + wl[3];
+        } else if ((tid & 31) == 0 && grp == 0) {
+            atomicAdd(a.loss, (double)l / (double)n);
+        }
+    }
+
+    // ---- tear-down: every TMEM read is complete before the warp frees it
+    umma::fence_before_sync();
+    __syncthreads();
+    if (!ok && tid == 0) atomicOr(&g_mlp_status, 1u);
+    if (warp == 0) umma::tmem_dealloc(tmem, tmem_cols<kTrain>());
+}
+
+__device__ __forceinline__ void adam_update(float *__restrict__ p, float gi, float *__restrict__ m,
+                                            float *__restrict__ v, int i, float lr, float beta1, float beta2, float eps,
+                                            float corr1, float corr2) {
+    const float mi = beta1 * m[i] + (1.0f - beta1) * gi;
+    const float vi = beta2 * v[i] + (1.0f - beta2) * gi * gi;
+    m[i] = mi;
+    v[i] = vi;
+    p[i] -= lr * (mi / corr1) / (sqrtf(vi / corr2) + eps);
+}
+__device__ __forceinline__ float average_update(float avg, float p, float decay) {
+    return fmaf(decay, avg - p, p); // decay avg + (1 - decay) p
+}
+
+// Adam step and weight average that follow a gradient (m null: none; avg null: none).
+struct AdamArgs {
+    float *net, *m, *v, *avg;
+    float lr, beta1, beta2, eps, corr1, corr2, decay;
+};
+
+// Deterministic reduction of the per-CTA gradient rows, column k summed over the
+// CTAs in CTA order (FP32, like the atomic path; the loss column in FP64), then
+// the Adam step and the average on it.  A block takes 32 columns: its
+// 8 warps bring the rows into shared memory, all in flight at once, and one
+// warp adds them.  (A thread per column that loaded its rows one after the other:
+// 8.5 us, and 4 us more for Adam and the average in launches of their own; now SSS.)
+constexpr int kSumThreads = 256;
+__global__ void __launch_bounds__(kSumThreads)
+    grad_sum_kernel(const float *__restrict__ partials, int ctas, int64_t n, float *__restrict__ grad,
+                    double *__restrict__ loss, const AdamArgs ad) {
+    __shared__ float s[kMaxGradCtas][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int k = blockIdx.x * 32 + lane;
+    if (k <= kParams) {
+#pragma unroll 8
+        for (int b = warp; b < ctas; b += kSumThreads / 32) s[b][lane] = __ldg(partials + (size_t)b * (kParams + 1) + k);
+    }
+    __syncthreads();
+    if (warp != 0) return;
     if (k < kParams) {
-        float s = 0.f;
-        for (int b = 0; b < ctas; ++b) s += partials[(size_t)b * (kParams + 1) + k];
-        grad[k] = s;
+        float g = 0.f;
+#pragma unroll 8
+        for (int b = 0; b < ctas; ++b) g += s[b][lane];
+        grad[k] = g;
+        if (ad.m) adam_update(ad.net, g, ad.m, ad.v, k, ad.lr, ad.beta1, ad.beta2, ad.eps, ad.corr1, ad.corr2);
+        if (ad.avg) ad.avg[k] = average_update(ad.avg[k], ad.net[k], ad.decay);
     } else if (k == kParams) {
-        double s = 0.0;
-        for (int b = 0; b < ctas; ++b) s += (double)partials[(size_t)b * (kParams + 1) + kParams];
-        *loss = s / (double)n;
+        double l = 0.0;
+        for (int b = 0; b < ctas; ++b) l += (double)s[b][lane];
+        *loss = l / (double)n;
     }
 }
 
@@ -599,19 +807,23 @@ __global__ void adam_kernel(float *__restrict__ p, const float *__restrict__ g, 
                             float corr1, float corr2) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
-    const float gi = g[i];
-    const float mi = beta1 * m[i] + (1.0f - beta1) * gi;
-    const float vi = beta2 * v[i] + (1.0f - beta2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    p[i] -= lr * (mi / corr1) / (sqrtf(vi / corr2) + eps);
+    adam_update(p, g[i], m, v, i, lr, beta1, beta2, eps, corr1, corr2);
 }
 
 __global__ void average_kernel(float *__restrict__ avg, const float *__restrict__ p, int count, float decay) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
-    avg[i] = fmaf(decay, avg[i] - p[i], p[i]); // decay avg + (1 - decay) p
+    avg[i] = average_update(avg[i], p[i], decay);
 }
+
+// The kernel and threads per CTA of a mode.
+template <int MODE>
+auto kernel_of() {
+    if constexpr (MODE == kTrain) return mlp_train_kernel;
+    else return mlp_kernel<MODE>;
+}
+template <int MODE>
+constexpr int kThreadsOf = MODE == kTrain ? kThreadsTrain : kThreadsMlp;
 
 // Resident CTAs per SM of a mode and the SM count, computed once per mode and
 // device from the device's limits: shared memory (with the per-block
@@ -626,12 +838,12 @@ int launch_shape(size_t smem, int &per_sm, int &sms) {
     int dev = 0;
     if (int e = cuda_check(cudaGetDevice(&dev), "cudaGetDevice")) return e;
     if (dev != cached_dev) {
-        if (int e = cuda_check(cudaFuncSetAttribute(mlp_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (int e = cuda_check(cudaFuncSetAttribute(kernel_of<MODE>(), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                     (int)smem),
                                "mlp smem attribute"))
             return e;
         cudaFuncAttributes fa{};
-        if (int e = cuda_check(cudaFuncGetAttributes(&fa, mlp_kernel<MODE>), "mlp attributes")) return e;
+        if (int e = cuda_check(cudaFuncGetAttributes(&fa, kernel_of<MODE>()), "mlp attributes")) return e;
         auto attr = [&](cudaDeviceAttr a, int fallback) {
             int v = 0;
             return (cudaDeviceGetAttribute(&v, a, dev) == cudaSuccess && v > 0) ? v : fallback;
@@ -643,10 +855,10 @@ int launch_shape(size_t smem, int &per_sm, int &sms) {
         const int threads_sm = attr(cudaDevAttrMaxThreadsPerMultiProcessor, 2048);
         const int blocks_sm = attr(cudaDevAttrMaxBlocksPerMultiprocessor, 32);
         const int regs_warp = ((fa.numRegs + 7) / 8) * 8 * 32;
-        const int warps = kThreadsMlp / 32;
+        const int warps = kThreadsOf<MODE> / 32;
         int n = smem_sm / ((int)smem + fa.sharedSizeBytes + reserved);
         n = std::min(n, regs_sm / (regs_warp * warps));
-        n = std::min(n, threads_sm / kThreadsMlp);
+        n = std::min(n, threads_sm / kThreadsOf<MODE>);
         n = std::min(n, blocks_sm);
         n = std::min(n, (int)(512u / tmem_cols<MODE>()));
         c_per_sm = n > 0 ? n : 1;
@@ -659,7 +871,7 @@ int launch_shape(size_t smem, int &per_sm, int &sms) {
 }
 
 template <int MODE>
-int launch(MlpArgs a, cudaStream_t st, int max_ctas = 0) {
+int launch(MlpArgs a, cudaStream_t st, int max_ctas = 0, const AdamArgs &ad = AdamArgs{}) {
     // training: one CTA per SM (its 256 TMEM columns and ~120 KB of shared memory)
     const size_t smem = MODE == kTrain ? (Layout<MODE>::bytes > (size_t)120 * 1024 ? Layout<MODE>::bytes
                                                                                      : (size_t)120 * 1024)
@@ -670,10 +882,10 @@ int launch(MlpArgs a, cudaStream_t st, int max_ctas = 0) {
     int64_t slots = (int64_t)sms * per_sm;
     if (max_ctas > 0 && slots > max_ctas) slots = max_ctas;
     const unsigned blocks = (unsigned)(tiles < slots ? tiles : slots);
-    mlp_kernel<MODE><<<blocks, kThreadsMlp, smem, st>>>(a);
+    kernel_of<MODE>()<<<blocks, kThreadsOf<MODE>, smem, st>>>(a);
     if (int e = cuda_check(cudaGetLastError(), "mlp launch")) return e;
     if (MODE == kTrain && a.partials) {
-        grad_sum_kernel<<<(kParams + 1 + 255) / 256, 256, 0, st>>>(a.partials, (int)blocks, a.n, a.grad, a.loss);
+        grad_sum_kernel<<<(kParams + 1 + 31) / 32, kSumThreads, 0, st>>>(a.partials, (int)blocks, a.n, a.grad, a.loss, ad);
         return cuda_check(cudaGetLastError(), "gradient sum launch");
     }
     return SSMD_OK;
@@ -737,6 +949,35 @@ extern "C" int ssmd_mlp_grad_ws(const float *net, const float *features, const f
     a.loss = loss;
     a.partials = workspace;
     return launch<kTrain>(a, reinterpret_cast<cudaStream_t>(stream), kMaxGradCtas);
+}
+
+extern "C" int ssmd_mlp_train_step(float *net, const float *features, const float *targets, const float *weights,
+                                   int64_t n_rows, const int64_t *rows, int64_t batch, float *grad, double *loss,
+                                   float *m, float *v, int64_t t, float lr, float beta1, float beta2, float eps,
+                                   float *avg, float decay, float *workspace, size_t workspace_bytes,
+                                   ssmd_stream_t stream) {
+    if (!net || !features || !targets || !rows || !grad || !loss || !m || !v || !workspace || n_rows <= 0 || batch <= 0 ||
+        t <= 0)
+        return fail(SSMD_ERR_INVALID_ARGUMENT, "null argument, n_rows <= 0, batch <= 0 or t <= 0");
+    if (batch > (int64_t)0x7FFFFFFF * kRows) return fail(SSMD_ERR_INVALID_ARGUMENT, "too many rows");
+    if (avg && !(decay >= 0.0f && decay <= 1.0f)) return fail(SSMD_ERR_INVALID_ARGUMENT, "decay outside [0, 1]");
+    if (workspace_bytes < ssmd_mlp_grad_workspace_bytes())
+        return fail(SSMD_ERR_INVALID_ARGUMENT, "workspace_bytes %zu < required %zu", workspace_bytes,
+                    ssmd_mlp_grad_workspace_bytes());
+    MlpArgs a{};
+    a.net = net;
+    a.feat = features;
+    a.target = targets;
+    a.weight = weights;
+    a.rows = rows;
+    a.n_rows = n_rows;
+    a.n = batch;
+    a.grad = grad;
+    a.loss = loss;
+    a.partials = workspace;
+    AdamArgs ad{net, m, v, avg, lr, beta1, beta2, eps, (float)(1.0 - pow((double)beta1, (double)t)),
+                (float)(1.0 - pow((double)beta2, (double)t)), decay};
+    return launch<kTrain>(a, reinterpret_cast<cudaStream_t>(stream), kMaxGradCtas, ad);
 }
 
 extern "C" int ssmd_closure_refresh(const ssmd_params *coarse, const LBMFields *fields, const float *net,
