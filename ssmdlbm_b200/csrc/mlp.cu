@@ -176,16 +176,25 @@ __device__ __forceinline__ void st8(unsigned char *tile, int r, int k0, int K, c
 }
 
 
-// Copy a [rows x K] block of fp32 weights (row stride K), times `scale` (a
-// power of two), into a bf16 tile of rows_pad rows (extra rows zero);
-// transpose: element (r, k) = src[k * rows + r].
-__device__ void load_weights(unsigned char *tile, const float *src, int rows, int rows_pad, int K, bool transpose,
-                             int tid, int threads, float scale = 1.0f) {
-    for (int e = tid; e < rows_pad * K; e += threads) {
-        const int r = e / K, k = e % K;
-        float v = 0.f;
-        if (r < rows) v = transpose ? src[k * rows + r] : src[r * K + k];
-        *reinterpret_cast<__nv_bfloat16 *>(tile + umma::kmajor_offset(r, k, K)) = __float2bfloat16_rn(v * scale);
+// Copy a [ROWS x K] block of fp32 weights (row stride K), times `scale` (a
+// power of two), into a bf16 tile of ROWS_PAD rows (extra rows zero); TRANS:
+// element (r, k) = src[k * ROWS + r].  A thread converts 8 values of a row and
+// stores them at once, and all its loads are in flight together: a CTA's
+// set-up is one round trip, not one per element of a thread (training kernel
+// on 65 536 rows, 4 tiles a CTA: 43 -> 40 us; forward of 1 M rows, 8 tiles a CTA: 75 ->
+// 67; refresh of 96 x 96 x 384 cells: 238 -> 229).
+template <int ROWS, int ROWS_PAD, int K, bool TRANS, int THREADS>
+__device__ __forceinline__ void load_weights(unsigned char *tile, const float *src, int tid, float scale = 1.0f) {
+    constexpr int CHUNKS = ROWS_PAD * (K / 8);
+#pragma unroll
+    for (int c0 = 0; c0 < CHUNKS; c0 += THREADS) {
+        const int c = c0 + tid;
+        if (CHUNKS % THREADS != 0 && c >= CHUNKS) break;
+        const int r = TRANS ? c % ROWS_PAD : c / (K / 8), k0 = 8 * (TRANS ? c / ROWS_PAD : c % (K / 8));
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = r < ROWS ? __ldg(src + (TRANS ? (k0 + i) * ROWS + r : r * K + k0 + i)) * scale : 0.f;
+        st8(tile, r, k0, K, v);
     }
 }
 
@@ -315,9 +324,9 @@ __global__ void __launch_bounds__(kThreadsMlp, 7) mlp_kernel(const MlpArgs a) {
         fence_barrier_init();
     }
     // W2 and W3 are fed with 2 gelu(z): halved weights, the same products
-    load_weights(sm + L::sW1, net + oW1, kH, kH, kK1, false, tid, kThreadsMlp);
-    load_weights(sm + L::sW2, net + oW2, kH, kH, kH, false, tid, kThreadsMlp, 0.5f);
-    load_weights(sm + L::sW3, net + oW3, kOut, kN3, kH, false, tid, kThreadsMlp, 0.5f);
+    load_weights<kH, kH, kK1, false, kThreadsMlp>(sm + L::sW1, net + oW1, tid);
+    load_weights<kH, kH, kH, false, kThreadsMlp>(sm + L::sW2, net + oW2, tid, 0.5f);
+    load_weights<kOut, kN3, kH, false, kThreadsMlp>(sm + L::sW3, net + oW3, tid, 0.5f);
     for (int e = tid; e < kH; e += kThreadsMlp) {
         b1[e] = net[oB1 + e];
         b2[e] = net[oB2 + e];
@@ -437,7 +446,7 @@ struct TrainRow {
 // kernel is a chain of MMA round trips and epilogues per tile; with one thread
 // per row (4 warps per SM, one per scheduler) the epilogues' ~5000 instructions
 // ran at the latency of one warp: 15 us a tile, 62 us for 65 536 rows; with four
-// threads per row LLL.  The rows of a mini-batch are read through their
+// threads per row 40, the gather included.  The rows of a mini-batch are read through their
 // indices (a.rows), the next tile's while this one's layers run: gathering them first took
 // three launches and 50 us of the 128 us step.  Every value and every sum is in
 // the order of one thread per row: the same bits.
@@ -497,10 +506,10 @@ __global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpAr
         *abort_flag = 0u;
         fence_barrier_init();
     }
-    load_weights(sm + L::sW1, net + oW1, kH, kH, kK1, false, tid, kThreadsTrain);
-    load_weights(sm + L::sW2, net + oW2, kH, kH, kH, false, tid, kThreadsTrain);
-    load_weights(sm + L::sW3, net + oW3, kOut, kN3, kH, false, tid, kThreadsTrain);
-    load_weights(sm + sW2T, net + oW2, kH, kH, kH, true, tid, kThreadsTrain); // (i, o) = W2[o][i]
+    load_weights<kH, kH, kK1, false, kThreadsTrain>(sm + L::sW1, net + oW1, tid);
+    load_weights<kH, kH, kH, false, kThreadsTrain>(sm + L::sW2, net + oW2, tid);
+    load_weights<kOut, kN3, kH, false, kThreadsTrain>(sm + L::sW3, net + oW3, tid);
+    load_weights<kH, kH, kH, true, kThreadsTrain>(sm + sW2T, net + oW2, tid); // (i, o) = W2[o][i]
     if (tid < kH) {
         b1[tid] = net[oB1 + tid];
         b2[tid] = net[oB2 + tid];
@@ -750,14 +759,12 @@ __global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpAr
     if (warp == 0) umma::tmem_dealloc(tmem, tmem_cols<kTrain>());
 }
 
-__device__ __forceinline__ void adam_update(float *__restrict__ p, float gi, float *__restrict__ m,
-                                            float *__restrict__ v, int i, float lr, float beta1, float beta2, float eps,
-                                            float corr1, float corr2) {
-    const float mi = beta1 * m[i] + (1.0f - beta1) * gi;
-    const float vi = beta2 * v[i] + (1.0f - beta2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    p[i] -= lr * (mi / corr1) / (sqrtf(vi / corr2) + eps);
+__device__ __forceinline__ void adam_update(float &p, float gi, float &m, float &v, float lr, float beta1, float beta2,
+                                            float eps, float corr1, float corr2) {
+    // (explicit fma: the kernels that share this round alike)
+    m = fmaf(1.0f - beta1, gi, beta1 * m);
+    v = fmaf((1.0f - beta2) * gi, gi, beta2 * v);
+    p -= lr * (m / corr1) / (sqrtf(v / corr2) + eps);
 }
 __device__ __forceinline__ float average_update(float avg, float p, float decay) {
     return fmaf(decay, avg - p, p); // decay avg + (1 - decay) p
@@ -774,7 +781,8 @@ struct AdamArgs {
 // the Adam step and the average on it.  A block takes 32 columns: its
 // 8 warps bring the rows into shared memory, all in flight at once, and one
 // warp adds them.  (A thread per column that loaded its rows one after the other:
-// 8.5 us, and 4 us more for Adam and the average in launches of their own; now SSS.)
+// 8.5 us, and 4 us more for Adam and the average in launches of their own; now 4.6 us
+// for all three.)
 constexpr int kSumThreads = 256;
 __global__ void __launch_bounds__(kSumThreads)
     grad_sum_kernel(const float *__restrict__ partials, int ctas, int64_t n, float *__restrict__ grad,
@@ -782,10 +790,18 @@ __global__ void __launch_bounds__(kSumThreads)
     __shared__ float s[kMaxGradCtas][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int k = blockIdx.x * 32 + lane;
-    if (k <= kParams) {
-#pragma unroll 8
-        for (int b = warp; b < ctas; b += kSumThreads / 32) s[b][lane] = __ldg(partials + (size_t)b * (kParams + 1) + k);
+    // Adam's operands are on their way while the rows come in
+    const bool step = warp == 0 && k < kParams;
+    const float m0 = step && ad.m ? ad.m[k] : 0.f, v0 = step && ad.m ? ad.v[k] : 0.f;
+    const float p0 = step && ad.net ? ad.net[k] : 0.f, a0 = step && ad.avg ? ad.avg[k] : 0.f;
+    float row[kMaxGradCtas / (kSumThreads / 32)];
+#pragma unroll
+    for (int i = 0; i < kMaxGradCtas / (kSumThreads / 32); ++i) {
+        const int b = warp + i * (kSumThreads / 32);
+        row[i] = b < ctas && k <= kParams ? __ldg(partials + (size_t)b * (kParams + 1) + k) : 0.f;
     }
+#pragma unroll
+    for (int i = 0; i < kMaxGradCtas / (kSumThreads / 32); ++i) s[warp + i * (kSumThreads / 32)][lane] = row[i];
     __syncthreads();
     if (warp != 0) return;
     if (k < kParams) {
@@ -793,8 +809,15 @@ __global__ void __launch_bounds__(kSumThreads)
 #pragma unroll 8
         for (int b = 0; b < ctas; ++b) g += s[b][lane];
         grad[k] = g;
-        if (ad.m) adam_update(ad.net, g, ad.m, ad.v, k, ad.lr, ad.beta1, ad.beta2, ad.eps, ad.corr1, ad.corr2);
-        if (ad.avg) ad.avg[k] = average_update(ad.avg[k], ad.net[k], ad.decay);
+        float p = p0;
+        if (ad.m) {
+            float m = m0, v = v0;
+            adam_update(p, g, m, v, ad.lr, ad.beta1, ad.beta2, ad.eps, ad.corr1, ad.corr2);
+            ad.net[k] = p;
+            ad.m[k] = m;
+            ad.v[k] = v;
+        }
+        if (ad.avg) ad.avg[k] = average_update(a0, p, ad.decay);
     } else if (k == kParams) {
         double l = 0.0;
         for (int b = 0; b < ctas; ++b) l += (double)s[b][lane];
@@ -807,7 +830,7 @@ __global__ void adam_kernel(float *__restrict__ p, const float *__restrict__ g, 
                             float corr1, float corr2) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
-    adam_update(p, g[i], m, v, i, lr, beta1, beta2, eps, corr1, corr2);
+    adam_update(p[i], g[i], m[i], v[i], lr, beta1, beta2, eps, corr1, corr2);
 }
 
 __global__ void average_kernel(float *__restrict__ avg, const float *__restrict__ p, int count, float decay) {
