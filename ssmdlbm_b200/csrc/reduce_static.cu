@@ -123,7 +123,7 @@ int reduce_static(const ssmd_params &p, const LBMFields &fl, uint64_t steps_done
     double *partials = scratch;
     double *result = scratch + (size_t)kRedVals * kStaticPartials;
     reduce_pass1<phase_t<T>><<<nb, kRedThreads, 0, st>>>(G, make_fields(fl), g, partials);
-    reduce_pass2<<<1, kRedThreads, 0, st>>>(partials, nb, result);
+    reduce_pass2<<<1, kFoldThreads, 0, st>>>(partials, nb, result);
     if (int e = cuda_check(cudaGetLastError(), "static reduce launch")) return e;
     if (int e = cuda_check(cudaMemcpyAsync(out_host, result, sizeof(double) * kRedVals,
                                            cudaMemcpyDeviceToHost, st),

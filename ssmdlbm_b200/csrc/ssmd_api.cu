@@ -85,7 +85,7 @@ int launch_reduce(const ssmd_params &p, const LBMFields &fl, uint64_t steps_done
     double *partials = reinterpret_cast<double *>(ws + kPartialOff);
     double *out = reinterpret_cast<double *>(ws + kRedOutOff);
     reduce_pass1<phase_t<T>><<<nb, kRedThreads, 0, st>>>(G, make_fields(fl), g, partials);
-    reduce_pass2<<<1, kRedThreads, 0, st>>>(partials, nb, out);
+    reduce_pass2<<<1, kFoldThreads, 0, st>>>(partials, nb, out);
     if (int e = cuda_check(cudaGetLastError(), "reduce launch")) return e;
     if (int e = cuda_check(cudaMemcpyAsync(out_host, out, sizeof(double) * kRedVals,
                                            cudaMemcpyDeviceToHost, st),

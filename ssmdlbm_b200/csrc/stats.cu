@@ -13,10 +13,13 @@
 //     a lock-free union-find: every label points at a smaller or equal index,
 //     unions hook the larger root under the smaller one with atomicMin
 //     (the GPU union-find of Playne and Hawick, IEEE TPDS 2018), then every
-//     label is compressed to its root (the smallest index of the component).
+//     label leads to its root (the smallest index of the component).
 //     Per component: cell count, FP64 sum of phi (the "volume"), and whether
 //     it touches the first fluid plane above the oil inlet.
 #include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstring>
 
 #include "host.cuh"
 
@@ -28,11 +31,11 @@ namespace {
 constexpr uint32_t kBG = 0xFFFFFFFFu;
 
 struct DropScratch {
-    uint32_t *label;
-    uint32_t *count;
-    double *volume;
-    uint32_t *touch;
-    uint32_t *n_out;
+    uint32_t *label;  // per cell: a smaller or equal cell of its component; kBG: background
+    uint32_t *cells;  // the foreground cells, unordered
+    uint32_t *count;  // per root: its component's cells, then its entry in the list
+    double *volume;   // per root
+    uint32_t *n_out;  // components found; n_out[1]: foreground cells
     ssmd_droplet *list;
     int max_list;
 };
@@ -60,15 +63,70 @@ __global__ void centreline_kernel(Geometry G, Fields F, float cx, float cy, doub
     phi_out[z] = n ? sp / n : 0.0;
 }
 
-__global__ void ccl_init(Geometry G, const float *phi, float thr, DropScratch S) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i >= G.cells) return;
-    const uint32_t c = (uint32_t)i;
-    const int x = c % G.nx, y = (c / G.nx) % G.ny, z = c / G.nxy;
-    S.label[c] = (fluid_cell(G, x, y, z) && phi[c] > thr) ? c : kBG;
-    S.count[c] = 0u;
-    S.volume[c] = 0.0;
-    S.touch[c] = 0u;
+// Labels, and the list of foreground cells: the kernels that follow visit only
+// those (a jet fills a few per cent of its lattice).  A block takes kCclCells
+// consecutive cells and reserves its part of the list with one atomic.  The
+// accumulators are cleared where a cell may become a root.  On 128 x 128 x 512 cells
+// labelling, clearing four arrays and scanning the lattice in each of four kernels took 201 us
+// (41 + 76 + 59 + 25); with the list DDD.
+constexpr int kCclThreads = 256, kCclPer = 8, kCclCells = kCclThreads * kCclPer;
+
+__global__ void __launch_bounds__(kCclThreads) ccl_init(Geometry G, const float *__restrict__ phi, float thr, DropScratch S) {
+    __shared__ uint32_t s_warp[kCclThreads / 32], s_base;
+    const uint64_t base = (uint64_t)blockIdx.x * kCclCells;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    float v[kCclPer];
+#pragma unroll
+    for (int k = 0; k < kCclPer; ++k) {
+        const uint64_t i = base + (uint64_t)k * kCclThreads + threadIdx.x;
+        v[k] = i < G.cells ? phi[i] : thr;
+    }
+    uint32_t on = 0, mine = 0; // this thread's foreground cells, and their number
+#pragma unroll
+    for (int k = 0; k < kCclPer; ++k) {
+        const uint64_t i = base + (uint64_t)k * kCclThreads + threadIdx.x;
+        const uint32_t c = (uint32_t)i;
+        bool fg = i < G.cells && v[k] > thr, first = false;
+        if (fg) {
+            const uint32_t zy = c / G.nx;
+            const int x = (int)(c - zy * G.nx), z = (int)(zy / G.ny), y = (int)(zy - (uint32_t)z * G.ny);
+            fg = fluid_cell(G, x, y, z);
+            first = x == 0;
+        }
+        // the label of a run of foreground cells of a row, within the warp's 32 cells: its first
+        const uint32_t run = __ballot_sync(0xffffffffu, fg);
+        const uint32_t starts = run & (~(run << 1) | __ballot_sync(0xffffffffu, fg && first));
+        if (i < G.cells) S.label[c] = fg ? c - (lane - (31u - __clz(starts & (0xffffffffu >> (31u - lane))))) : kBG;
+        if (fg) {
+            on |= 1u << k;
+            ++mine;
+            S.count[c] = 0u;
+            S.volume[c] = 0.0;
+        }
+    }
+    // exclusive scan of `mine` over the block
+    uint32_t scan = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, scan, o);
+        if (lane >= (uint32_t)o) scan += t;
+    }
+    if (lane == 31u) s_warp[warp] = scan;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t t = 0;
+        for (int w = 0; w < kCclThreads / 32; ++w) {
+            const uint32_t k = s_warp[w];
+            s_warp[w] = t;
+            t += k;
+        }
+        s_base = t ? atomicAdd(S.n_out + 1, t) : 0u;
+    }
+    __syncthreads();
+    uint32_t at = s_base + s_warp[warp] + scan - mine;
+#pragma unroll
+    for (int k = 0; k < kCclPer; ++k)
+        if (on & (1u << k)) S.cells[at++] = (uint32_t)(base + (uint64_t)k * kCclThreads + threadIdx.x);
 }
 
 __device__ __forceinline__ uint32_t find_root(const uint32_t *L, uint32_t a) {
@@ -97,54 +155,98 @@ __device__ __forceinline__ void unite(uint32_t *L, uint32_t a, uint32_t b) {
     }
 }
 
+// Unions with the next cell along x, y and z, left out where they follow from
+// others: along x inside a run that ccl_init labelled, along y and z where the pair
+// one x to the left is foreground too (it is united, and both its cells are with ours).
+// With every foreground pair united (long chains on a few labels) this took 63 of the
+// 111 us; now UUU.
 __global__ void ccl_union(Geometry G, DropScratch S) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i >= G.cells) return;
-    const uint32_t c = (uint32_t)i;
-    if (S.label[c] == kBG) return;
-    const int x = c % G.nx, y = (c / G.nx) % G.ny, z = c / G.nxy;
-    const int nb[3][3] = {{x + 1, y, z}, {x, y + 1, z}, {x, y, z + 1}};
-    const bool per[3] = {G.bcx == BC_PERIODIC, G.bcy == BC_PERIODIC, G.bcz == BC_PERIODIC};
-    const int n[3] = {(int)G.nx, (int)G.ny, (int)G.nz};
-    for (int d = 0; d < 3; ++d) {
-        int q[3] = {nb[d][0], nb[d][1], nb[d][2]};
-        if (q[d] >= n[d]) {
-            if (!per[d]) continue;
-            q[d] -= n[d];
+    const uint32_t total = S.n_out[1];
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t c = S.cells[i];
+        const uint32_t zy = c / G.nx;
+        const int x = (int)(c - zy * G.nx), z = (int)(zy / G.ny), y = (int)(zy - (uint32_t)z * G.ny);
+        const bool left = x > 0 && S.label[c - 1] != kBG;
+        const bool per[3] = {G.bcx == BC_PERIODIC, G.bcy == BC_PERIODIC, G.bcz == BC_PERIODIC};
+        const int n[3] = {(int)G.nx, (int)G.ny, (int)G.nz};
+        for (int d = 0; d < 3; ++d) {
+            int q[3] = {x, y, z};
+            q[d] += 1;
+            const bool wraps = q[d] >= n[d];
+            if (wraps) {
+                if (!per[d]) continue;
+                q[d] -= n[d];
+            }
+            if (d == 0 && !wraps && (c & 31u) != 31u) continue; // the run's label, or no neighbour
+            const uint32_t j = cell_index(G, q[0], q[1], q[2]);
+            if (S.label[j] == kBG) continue; // (background or outside the fluid region)
+            if (d > 0 && left && S.label[j - 1] != kBG) continue;
+            unite(S.label, c, j);
         }
-        if (!fluid_cell(G, q[0], q[1], q[2])) continue;
-        const uint32_t j = cell_index(G, q[0], q[1], q[2]);
-        if (S.label[j] == kBG) continue;
-        unite(S.label, c, j);
     }
 }
 
-__global__ void ccl_compress_accumulate(Geometry G, const float *phi, DropScratch S) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i >= G.cells) return;
-    const uint32_t c = (uint32_t)i;
-    if (S.label[c] == kBG) return;
-    const uint32_t r = find_root(S.label, c);
-    atomicAdd(&S.count[r], 1u);
-    atomicAdd(&S.volume[r], (double)phi[c]);
-    if ((int)(c / G.nxy) == G.z_lo) S.touch[r] = 1u;
+// Cells and volume per root.  Neighbouring entries of the list mostly belong to
+// one component: a warp whose cells all do adds its sums with one atomic each (a
+// jet's one component took an atomic per cell on one address).
+__global__ void ccl_accumulate(Geometry G, const float *__restrict__ phi, DropScratch S) {
+    const uint32_t total = S.n_out[1];
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); i0 < total; i0 += stride) { // (warp-uniform)
+        const uint64_t i = i0 + lane;
+        const bool on = i < total;
+        uint32_t r = 0;
+        double vol = 0.0;
+        if (on) {
+            const uint32_t c = S.cells[i];
+            r = find_root(S.label, c);
+            vol = (double)phi[c];
+        }
+        const uint32_t active = __ballot_sync(0xffffffffu, on);
+        const uint32_t r0 = __shfl_sync(0xffffffffu, r, 0); // (lane 0 is on whenever any lane is)
+        if (__all_sync(0xffffffffu, !on || r == r0)) {
+            for (int o = 16; o > 0; o >>= 1) vol += __shfl_xor_sync(0xffffffffu, vol, o);
+            if (lane == 0) {
+                atomicAdd(&S.count[r0], (uint32_t)__popc(active));
+                atomicAdd(&S.volume[r0], vol);
+            }
+        } else if (on) {
+            atomicAdd(&S.count[r], 1u);
+            atomicAdd(&S.volume[r], vol);
+        }
+    }
 }
 
-__global__ void ccl_collect(Geometry G, DropScratch S) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i >= G.cells) return;
-    const uint32_t c = (uint32_t)i;
-    const uint32_t n = S.count[c];
-    if (n == 0u) return;
-    const uint32_t slot_i = atomicAdd(S.n_out, 1u);
-    if ((int)slot_i >= S.max_list) return;
-    ssmd_droplet d;
-    d.root = c;
-    d.cells = n;
-    d.volume = S.volume[c];
-    d.touches_inlet = S.touch[c];
-    d.reserved = 0u;
-    S.list[slot_i] = d;
+// A list entry per root; its index replaces the root's count (max_list when the
+// list is full), for ccl_touch.
+__global__ void ccl_collect(DropScratch S) {
+    const uint32_t total = S.n_out[1];
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t c = S.cells[i];
+        if (S.label[c] != c) continue;
+        const uint32_t slot_i = atomicAdd(S.n_out, 1u);
+        const uint32_t cells = S.count[c];
+        S.count[c] = slot_i;
+        if (slot_i >= (uint32_t)S.max_list) continue;
+        ssmd_droplet d;
+        d.root = c;
+        d.cells = cells;
+        d.volume = S.volume[c];
+        d.touches_inlet = 0u;
+        d.reserved = 0u;
+        S.list[slot_i] = d;
+    }
+}
+
+// Components with a cell in the first fluid plane.
+__global__ void ccl_touch(Geometry G, DropScratch S) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= G.nxy) return;
+    const uint32_t c = (uint32_t)G.z_lo * G.nxy + i;
+    if (S.label[c] == kBG) return;
+    const uint32_t slot_i = S.count[find_root(S.label, c)];
+    if (slot_i < (uint32_t)S.max_list) S.list[slot_i].touches_inlet = 1u;
 }
 
 size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -155,25 +257,29 @@ size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
 // through the fluid slots (q, x) whose x + c_q is a ghost cell.  FP64 sums;
 // with the collision conserving phi per cell this closes the budget
 // sum phi^{n+1} = sum phi^n + inflow - outflow.
+// Only the fluid cells beside a ghost layer take part, so only those planes are
+// visited: blockIdx.y = 2 axis + side, first index along the face's first axis (scanning
+// every cell for them took 82 us on 128 x 128 x 512 cells; the faces take FFF).
 template <class TG>
 __global__ void phase_flux_kernel(Geometry G, const TG *g, double *acc) {
     __shared__ double s_in[256], s_out[256];
     double in = 0.0, out = 0.0;
-    const bool per[3] = {G.bcx == BC_PERIODIC, G.bcy == BC_PERIODIC, G.bcz == BC_PERIODIC};
-    const int n[3] = {(int)G.nx, (int)G.ny, (int)G.nz};
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < G.cells;
+    const int axis = (int)blockIdx.y >> 1, side = (int)blockIdx.y & 1;
+    const bool per = axis == 0 ? G.bcx == BC_PERIODIC : (axis == 1 ? G.bcy == BC_PERIODIC : G.bcz == BC_PERIODIC);
+    if (per) return; // (the whole block)
+    const int lo[3] = {G.x_lo, G.y_lo, G.z_lo}, hi[3] = {G.x_hi, G.y_hi, G.z_hi};
+    const uint32_t step[3] = {1u, G.nx, G.nxy};
+    const int a0 = axis == 0 ? 1 : 0, a1 = axis == 2 ? 1 : 2;
+    const uint32_t n0 = (uint32_t)(hi[a0] - lo[a0] + 1), n1 = (uint32_t)(hi[a1] - lo[a1] + 1);
+    const int q_out = 2 * axis + (side ? 1 : 2), q_in = 2 * axis + (side ? 2 : 1); // 1:+x 2:-x 3:+y 4:-y 5:+z 6:-z
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < (uint64_t)n0 * n1;
          i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t c = (uint32_t)i;
-        const int p[3] = {(int)(c % G.nx), (int)((c / G.nx) % G.ny), (int)(c / G.nxy)};
-        if (!fluid_cell(G, p[0], p[1], p[2])) continue;
-        for (int q = 1; q < 7; ++q) {
-            const int axis = (q - 1) >> 1, sgn = (q & 1) ? 1 : -1; // 1:+x 2:-x 3:+y 4:-y 5:+z 6:-z
-            int a[3] = {p[0], p[1], p[2]}, b[3] = {p[0], p[1], p[2]};
-            a[axis] = axis_nb(p[axis] - sgn, n[axis], per[axis]); // source of direction q
-            b[axis] = axis_nb(p[axis] + sgn, n[axis], per[axis]); // where this cell's q goes
-            if (!fluid_cell(G, a[0], a[1], a[2])) in += (double)Store<TG>::ld(g + slot(G, q, cell_index(G, a[0], a[1], a[2])));
-            if (!fluid_cell(G, b[0], b[1], b[2])) out += (double)Store<TG>::ld(g + slot(G, q, c));
-        }
+        const uint32_t i1 = (uint32_t)(i / n0), i0 = (uint32_t)(i - (uint64_t)i1 * n0);
+        const uint32_t c = (uint32_t)(side ? hi[axis] : lo[axis]) * step[axis] + (lo[a0] + i0) * step[a0] +
+                           (lo[a1] + i1) * step[a1];
+        const uint32_t ghost = side ? c + step[axis] : c - step[axis];
+        in += (double)Store<TG>::ld(g + slot(G, q_in, ghost));
+        out += (double)Store<TG>::ld(g + slot(G, q_out, c));
     }
     s_in[threadIdx.x] = in;
     s_out[threadIdx.x] = out;
@@ -226,9 +332,9 @@ extern "C" int ssmd_droplets(const ssmd_params *p, const LBMFields *fields, floa
     DropScratch S{};
     S.label = reinterpret_cast<uint32_t *>(s);
     s += round256(n * 4);
-    S.count = reinterpret_cast<uint32_t *>(s);
+    S.cells = reinterpret_cast<uint32_t *>(s);
     s += round256(n * 4);
-    S.touch = reinterpret_cast<uint32_t *>(s);
+    S.count = reinterpret_cast<uint32_t *>(s);
     s += round256(n * 4);
     S.volume = reinterpret_cast<double *>(s);
     s += round256(n * 8);
@@ -237,20 +343,30 @@ extern "C" int ssmd_droplets(const ssmd_params *p, const LBMFields *fields, floa
     S.list = reinterpret_cast<ssmd_droplet *>(s);
     S.max_list = max_droplets;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const unsigned nb = (unsigned)((n + 255) / 256);
-    if (int e = cuda_check(cudaMemsetAsync(S.n_out, 0, sizeof(uint32_t), st), "droplet counter")) return e;
-    ccl_init<<<nb, 256, 0, st>>>(G, fields->phi, threshold, S);
+    if (int e = cuda_check(cudaMemsetAsync(S.n_out, 0, 2 * sizeof(uint32_t), st), "droplet counters")) return e;
+    ccl_init<<<(unsigned)((n + kCclCells - 1) / kCclCells), kCclThreads, 0, st>>>(G, fields->phi, threshold, S);
+    const unsigned nb = (unsigned)std::min<size_t>((n + 255) / 256, 8 * 148); // (grid-stride over the list)
     ccl_union<<<nb, 256, 0, st>>>(G, S);
-    ccl_compress_accumulate<<<nb, 256, 0, st>>>(G, fields->phi, S);
-    ccl_collect<<<nb, 256, 0, st>>>(G, S);
+    ccl_accumulate<<<nb, 256, 0, st>>>(G, fields->phi, S);
+    ccl_collect<<<nb, 256, 0, st>>>(S);
+    ccl_touch<<<(G.nxy + 255) / 256, 256, 0, st>>>(G, S);
     if (int e = cuda_check(cudaGetLastError(), "droplet kernels")) return e;
-    uint32_t found = 0;
-    if (int e = cuda_check(cudaMemcpyAsync(&found, S.n_out, sizeof found, cudaMemcpyDeviceToHost, st), "count"))
+    // the number found and the first entries in one read (the list follows its header)
+    constexpr int kFirst = 256;
+    const int32_t first = max_droplets < kFirst ? max_droplets : kFirst;
+    alignas(16) char head[256 + kFirst * sizeof(ssmd_droplet)];
+    if (int e = cuda_check(cudaMemcpyAsync(head, S.n_out, 256 + (size_t)first * sizeof(ssmd_droplet),
+                                           cudaMemcpyDeviceToHost, st),
+                           "droplet list"))
         return e;
     if (int e = cuda_check(cudaStreamSynchronize(st), "droplet sync")) return e;
+    uint32_t found = 0;
+    std::memcpy(&found, head, sizeof found);
     const int32_t k = (int32_t)(found < (uint32_t)max_droplets ? found : (uint32_t)max_droplets);
-    if (k > 0) {
-        if (int e = cuda_check(cudaMemcpyAsync(out, S.list, sizeof(ssmd_droplet) * k, cudaMemcpyDeviceToHost, st),
+    std::memcpy(out, head + 256, sizeof(ssmd_droplet) * (size_t)std::min(k, first));
+    if (k > first) {
+        if (int e = cuda_check(cudaMemcpyAsync(out + first, S.list + first, sizeof(ssmd_droplet) * (size_t)(k - first),
+                                               cudaMemcpyDeviceToHost, st),
                                "droplet list"))
             return e;
         if (int e = cuda_check(cudaStreamSynchronize(st), "droplet sync")) return e;
@@ -271,8 +387,8 @@ extern "C" int ssmd_phase_flux(const ssmd_params *p, const LBMFields *fields, ui
     double *acc = reinterpret_cast<double *>(static_cast<char *>(p->workspace) + kPartialOff);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (int e = cuda_check(cudaMemsetAsync(acc, 0, 2 * sizeof(double), st), "flux clear")) return e;
-    uint64_t nb64 = (G.cells + 255) / 256;
-    const unsigned nb = (unsigned)(nb64 < 4096 ? nb64 : 4096);
+    const uint64_t face = std::max({(uint64_t)G.nx * G.ny, (uint64_t)G.nx * G.nz, (uint64_t)G.ny * G.nz});
+    const dim3 nb((unsigned)std::min<uint64_t>((face + 255) / 256, 512), 6);
     switch (p->storage) {
     case SSMD_STORAGE_F32: phase_flux_kernel<float><<<nb, 256, 0, st>>>(G, static_cast<const float *>(g), acc); break;
     case SSMD_STORAGE_F16: phase_flux_kernel<__half><<<nb, 256, 0, st>>>(G, static_cast<const __half *>(g), acc); break;

@@ -195,21 +195,24 @@ class Simulation:
         self.sync()
         return uz.cpu().numpy(), phi.cpu().numpy()
 
+    _DROPLET = np.dtype([("root", "u4"), ("cells", "u4"), ("volume", "f8"), ("touches_inlet", "u4"), ("reserved", "u4")])
+
     def droplets(self, threshold: float = 0.5, max_droplets: int = 100000) -> np.ndarray:
         """Connected components of phi > threshold (structured array sorted by
         root: root, cells, volume, touches_inlet).  Needs store_macros fields."""
         L = lib()
         nbytes = int(L.ssmd_droplets_scratch_bytes(ctypes.byref(self.p), max_droplets))
         scratch = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
-        out = (_lib.Droplet * max_droplets)()
+        out = np.empty(max(1, max_droplets), dtype=self._DROPLET)  # struct ssmd_droplet
         n = ctypes.c_int32()
         torch.cuda.synchronize(self.device)
         check(L.ssmd_droplets(ctypes.byref(self.p), ctypes.byref(self.fields), threshold, scratch.data_ptr(),
-                              nbytes, out, max_droplets, ctypes.byref(n), self.stream))
+                              nbytes, out.ctypes.data_as(ctypes.POINTER(_lib.Droplet)), max_droplets, ctypes.byref(n),
+                              self.stream))
         k = min(n.value, max_droplets)
         arr = np.zeros(k, dtype=[("root", "u4"), ("cells", "u4"), ("volume", "f8"), ("touches_inlet", "u4")])
-        for i in range(k):
-            arr[i] = (out[i].root, out[i].cells, out[i].volume, out[i].touches_inlet)
+        for name in arr.dtype.names:
+            arr[name] = out[name][:k]
         arr.sort(order="root")
         return arr
 
