@@ -68,7 +68,7 @@ __global__ void centreline_kernel(Geometry G, Fields F, float cx, float cy, doub
 // consecutive cells and reserves its part of the list with one atomic.  The
 // accumulators are cleared where a cell may become a root.  On 128 x 128 x 512 cells
 // labelling, clearing four arrays and scanning the lattice in each of four kernels took 201 us
-// (41 + 76 + 59 + 25); with the list DDD.
+// (41 + 76 + 59 + 25); with the list 69 (20 + 28 + 15 + 3 + 3).
 constexpr int kCclThreads = 256, kCclPer = 8, kCclCells = kCclThreads * kCclPer;
 
 __global__ void __launch_bounds__(kCclThreads) ccl_init(Geometry G, const float *__restrict__ phi, float thr, DropScratch S) {
@@ -158,8 +158,8 @@ __device__ __forceinline__ void unite(uint32_t *L, uint32_t a, uint32_t b) {
 // Unions with the next cell along x, y and z, left out where they follow from
 // others: along x inside a run that ccl_init labelled, along y and z where the pair
 // one x to the left is foreground too (it is united, and both its cells are with ours).
-// With every foreground pair united (long chains on a few labels) this took 63 of the
-// 111 us; now UUU.
+// With every foreground pair united (long chains on a few labels) this took 63 us,
+// now 28.
 __global__ void ccl_union(Geometry G, DropScratch S) {
     const uint32_t total = S.n_out[1];
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
@@ -259,7 +259,7 @@ size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
 // sum phi^{n+1} = sum phi^n + inflow - outflow.
 // Only the fluid cells beside a ghost layer take part, so only those planes are
 // visited: blockIdx.y = 2 axis + side, first index along the face's first axis (scanning
-// every cell for them took 82 us on 128 x 128 x 512 cells; the faces take FFF).
+// every cell for them took 82 us on 128 x 128 x 512 cells; the faces take 4.6).
 template <class TG>
 __global__ void phase_flux_kernel(Geometry G, const TG *g, double *acc) {
     __shared__ double s_in[256], s_out[256];
