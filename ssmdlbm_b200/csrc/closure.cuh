@@ -21,36 +21,9 @@ inline Grid grid_of(const ssmd_params &p) {
                 p.bc_z == SSMD_BC_PERIODIC};
 }
 
-__device__ __forceinline__ int nbr(int c, int d, int n, bool per) {
-    int v = c + d;
-    if (per) v = v < 0 ? v + n : (v >= n ? v - n : v);
-    else v = v < 0 ? 0 : (v >= n ? n - 1 : v);
-    return v;
-}
-
-__device__ __forceinline__ int64_t idx(const Grid &g, int x, int y, int z) {
-    return (int64_t)x + (int64_t)g.nx * ((int64_t)y + (int64_t)g.ny * z);
-}
-
-// Central-difference gradient of a scalar array at (x, y, z).
-__device__ __forceinline__ void grad3(const Grid &g, const float *a, int x, int y, int z, float &gx, float &gy,
-                                      float &gz) {
-    gx = 0.5f * (a[idx(g, nbr(x, 1, g.nx, g.px), y, z)] - a[idx(g, nbr(x, -1, g.nx, g.px), y, z)]);
-    gy = 0.5f * (a[idx(g, x, nbr(y, 1, g.ny, g.py), z)] - a[idx(g, x, nbr(y, -1, g.ny, g.py), z)]);
-    gz = 0.5f * (a[idx(g, x, y, nbr(z, 1, g.nz, g.pz))] - a[idx(g, x, y, nbr(z, -1, g.nz, g.pz))]);
-}
-
-// Velocity gradient d[i][j] = d u_i / d x_j and the strain rate S = (d + d^T)/2.
-__device__ __forceinline__ void strain(const Grid &g, const float *ux, const float *uy, const float *uz, int x,
-                                       int y, int z, float (&d)[3][3]) {
-    grad3(g, ux, x, y, z, d[0][0], d[0][1], d[0][2]);
-    grad3(g, uy, x, y, z, d[1][0], d[1][1], d[1][2]);
-    grad3(g, uz, x, y, z, d[2][0], d[2][1], d[2][2]);
-}
-
 // The six face neighbours of a cell, as 32-bit cell indices (a lattice has
-// fewer than 2^32 cells): the same cells nbr() and idx() give, found with one
-// 32-bit division chain per cell instead of 64-bit arithmetic per load.
+// fewer than 2^32 cells), found with one 32-bit division chain per cell instead
+// of 64-bit arithmetic per load.
 struct Faces {
     uint32_t xp, xm, yp, ym, zp, zm;
 };
@@ -58,7 +31,7 @@ struct Faces {
 __device__ __forceinline__ Faces faces(const Grid &g, uint32_t c) {
     const uint32_t nx = (uint32_t)g.nx, nxy = nx * (uint32_t)g.ny;
     const uint32_t z = c / nxy, rxy = c - z * nxy, y = rxy / nx, x = rxy - y * nx;
-    // step d along an axis of n cells at coordinate v, stride s: wrap or clamp like nbr()
+    // step along an axis of n cells at coordinate v, stride s: wraps on a periodic axis, clamps at the face of another
     auto up = [](uint32_t v, uint32_t n, uint32_t s, bool per) { return v + 1 < n ? s : (per ? s - n * s : 0u); };
     auto dn = [](uint32_t v, uint32_t n, uint32_t s, bool per) { return v > 0 ? 0u - s : (per ? n * s - s : 0u); };
     Faces f;
