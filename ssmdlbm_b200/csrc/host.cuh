@@ -137,22 +137,55 @@ inline Averages make_averages(const ssmd_params &p) {
     return A;
 }
 
-// Running means at cells the bulk kernel does not update (ghost layers), from
-// the macroscopic fields the boundary kernels wrote; t = avg_t + 1.
-static __global__ void averages_kernel(Geometry G, Fields F, Averages A, const DeviceStatus *status,
-                                       int ghost_only) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i >= G.cells) return;
-    if (ghost_only) {
-        const uint32_t c = (uint32_t)i;
-        const int x = c % G.nx, y = (c / G.nx) % G.ny, z = c / G.nxy;
-        if (x >= G.x_lo && x <= G.x_hi && y >= G.y_lo && y <= G.y_hi && z >= G.z_lo && z <= G.z_hi) return;
-    }
+// Running means from the macroscopic fields, t = avg_t + 1, after which the last
+// block advances avg_t.  GHOST: only the cells the bulk kernel does not update, whose
+// fields the boundary kernels wrote: blockIdx.y = 2 axis + side, the ghost plane's cells
+// that no earlier axis has (z planes whole, y planes at fluid z, x planes at fluid y and
+// z).  Scanning the whole lattice for them took 13 us on 96 x 96 x 192 cells, and the
+// advance a launch of its own; now 5.
+template <bool GHOST>
+static __global__ void averages_kernel(Geometry G, Fields F, Averages A, DeviceStatus *status) {
     const float t = (float)(status->avg_t + 1u);
-    accumulate_averages(A, i, t, F.phi[i], F.ux[i], F.uy[i], F.uz[i]);
+    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if constexpr (!GHOST) {
+        if (i < G.cells) accumulate_averages_together(A, i, t, F.phi[i], F.ux[i], F.uy[i], F.uz[i]);
+    } else {
+        const int face = (int)blockIdx.y, side = face & 1;
+        const bool ghosts = face < 2 ? G.x_lo > 0 : (face < 4 ? G.y_lo > 0 : G.z_lo > 0);
+        const uint32_t fy = (uint32_t)(G.y_hi - G.y_lo + 1), fz = (uint32_t)(G.z_hi - G.z_lo + 1);
+        const uint32_t n0 = face < 2 ? fy : G.nx, n1 = face < 4 ? fz : G.ny;
+        if (ghosts && i < (uint64_t)n0 * n1) {
+            const uint32_t i1 = (uint32_t)(i / n0), i0 = (uint32_t)(i - (uint64_t)i1 * n0);
+            uint32_t x, y, z;
+            if (face < 2) x = side ? G.nx - 1 : 0u, y = G.y_lo + i0, z = G.z_lo + i1;
+            else if (face < 4) x = i0, y = side ? G.ny - 1 : 0u, z = G.z_lo + i1;
+            else x = i0, y = i1, z = side ? G.nz - 1 : 0u;
+            const uint32_t c = cell_index(G, x, y, z);
+            accumulate_averages_together(A, c, t, F.phi[c], F.ux[c], F.uy[c], F.uz[c]);
+        }
+    }
+    __syncthreads(); // every thread has read avg_t
+    if (threadIdx.x == 0) {
+        const unsigned blocks = gridDim.x * gridDim.y;
+        if (atomicAdd(&status->work_next, 1u) == blocks - 1u) { // every block has
+            status->work_next = 0u;
+            status->avg_t += 1u;
+        }
+    }
 }
 
-static __global__ void advance_avg_kernel(DeviceStatus *status) { status->avg_t += 1u; }
+inline void launch_averages(const Geometry &G, const Fields &F, const Averages &A, DeviceStatus *status, bool ghost_only,
+                            cudaStream_t st) {
+    if (!ghost_only) {
+        averages_kernel<false><<<(unsigned)((G.cells + 255) / 256), 256, 0, st>>>(G, F, A, status);
+        return;
+    }
+    uint64_t most = 1;
+    if (G.x_lo > 0) most = std::max(most, (uint64_t)G.ny * G.nz);
+    if (G.y_lo > 0) most = std::max(most, (uint64_t)G.nx * G.nz);
+    if (G.z_lo > 0) most = std::max(most, (uint64_t)G.nx * G.ny);
+    averages_kernel<true><<<dim3((unsigned)((most + 255) / 256), 6), 256, 0, st>>>(G, F, A, status);
+}
 
 // Dynamic shared memory of a bulk instantiation (TMA boxes or slabs).
 template <int Q, class T, int PATH>
@@ -163,7 +196,7 @@ constexpr size_t bulk_dyn_smem() {
 // Resident bulk work items per SM for this instantiation (queried once per
 // device and kernel, after raising its dynamic shared-memory limit) and the
 // SM count.
-template <int Q, class T, int PATH, bool PXY = false>
+template <int Q, class T, int PATH, bool PXY = false, bool AVG = false>
 inline void bulk_slots(int &per_sm, int &sms) {
     static thread_local int cached_dev = -1, cached_per_sm = 0, cached_sms = 0;
     int dev = 0;
@@ -172,9 +205,9 @@ inline void bulk_slots(int &per_sm, int &sms) {
         int n = 0, m = 0;
         const size_t dyn = bulk_dyn_smem<Q, T, PATH>();
         if (dyn > 0)
-            cudaFuncSetAttribute(bulk_kernel<Q, T, phase_t<T>, PATH, PXY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(bulk_kernel<Q, T, phase_t<T>, PATH, PXY, AVG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)dyn);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bulk_kernel<Q, T, phase_t<T>, PATH, PXY>, kThreads, dyn) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bulk_kernel<Q, T, phase_t<T>, PATH, PXY, AVG>, kThreads, dyn) !=
             cudaSuccess)
             n = 1;
         if (cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) m = 148;
@@ -316,12 +349,14 @@ int launch_step(const ssmd_params &p, const LBMFields &fl, uint64_t step, uint32
         !(encode_populations<TG>(&gmap, a.g_src, a.geo.nx, a.geo.ny, a.geo.nz, 7, Slab<TG>::WX, kTY) &&
           encode_populations<T>(&fmap, a.f_src, a.geo.nx, a.geo.ny, a.geo.nz, Q, Slab<T>::WX, kTY)))
         return fail(SSMD_ERR_UNSUPPORTED, "slab path needs nx * element size to be a multiple of 16 bytes");
-    const bool pxy = a.geo.bcx == BC_PERIODIC && a.geo.bcy == BC_PERIODIC;
+    const bool pxy = a.geo.bcx == BC_PERIODIC && a.geo.bcy == BC_PERIODIC, avg = flags & SSMD_STEP_AVERAGE;
     int per_sm = 1, sms = 1;
     if (path == SSMD_PATH_TMA) bulk_slots<Q, T, 2>(per_sm, sms);
     else if (path == SSMD_PATH_SLAB) {
         if constexpr (kSlabs) bulk_slots<Q, T, 3>(per_sm, sms);
-    } else if (pxy) bulk_slots<Q, T, 1, true>(per_sm, sms);
+    } else if (pxy && avg) bulk_slots<Q, T, 1, true, true>(per_sm, sms);
+    else if (pxy) bulk_slots<Q, T, 1, true>(per_sm, sms);
+    else if (avg) bulk_slots<Q, T, 1, false, true>(per_sm, sms);
     else bulk_slots<Q, T, 1>(per_sm, sms);
     tiling(p, a.geo, per_sm * sms, sms, a.tiles_x, a.tiles_y, a.zchunk, a.nzchunks);
     a.halo_mod = (a.geo.bcx == BC_PERIODIC && a.geo.nx < (uint32_t)(kTX + 4)) ||
@@ -336,9 +371,14 @@ int launch_step(const ssmd_params &p, const LBMFields &fl, uint64_t step, uint32
     if (path == SSMD_PATH_TMA)
         bulk_kernel<Q, T, TG, 2><<<nblk, blk, bulk_dyn_smem<Q, T, 2>(), st>>>(a, gmap, fmap);
     else if (path == SSMD_PATH_SLAB) {
-        if constexpr (kSlabs) bulk_kernel<Q, T, TG, 3><<<nblk, blk, bulk_dyn_smem<Q, T, 3>(), st>>>(a, gmap, fmap);
-    } else if (pxy)
+        if constexpr (kSlabs)
+            bulk_kernel<Q, T, TG, 3><<<nblk, blk, bulk_dyn_smem<Q, T, 3>(), st>>>(a, gmap, fmap);
+    } else if (pxy && avg)
+        bulk_kernel<Q, T, TG, 1, true, true><<<nblk, blk, 0, st>>>(a, gmap, fmap);
+    else if (pxy)
         bulk_kernel<Q, T, TG, 1, true><<<nblk, blk, 0, st>>>(a, gmap, fmap);
+    else if (avg)
+        bulk_kernel<Q, T, TG, 1, false, true><<<nblk, blk, 0, st>>>(a, gmap, fmap);
     else
         bulk_kernel<Q, T, TG, 1><<<nblk, blk, 0, st>>>(a, gmap, fmap);
     if (ev1) cudaEventRecord(ev1, st);
@@ -355,9 +395,7 @@ int launch_step(const ssmd_params &p, const LBMFields &fl, uint64_t step, uint32
     if (G.bcy == BC_COPY) faces(ic<BK_COPY_Y>{}, G.nx, G.nz);
     if (flags & SSMD_STEP_AVERAGE) {
         // the bulk kernel updated the fluid cells; the ghost layers follow, then t advances
-        const unsigned nb = (unsigned)((G.cells + 255) / 256);
-        averages_kernel<<<nb, 256, 0, st>>>(G, a.fld, a.avg, a.status, 1);
-        advance_avg_kernel<<<1, 1, 0, st>>>(a.status);
+        launch_averages(G, a.fld, a.avg, a.status, true, st);
     }
     return cuda_check(cudaGetLastError(), "boundary kernel launch");
 }
