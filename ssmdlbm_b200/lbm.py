@@ -187,13 +187,14 @@ class Simulation:
             p = self.p.copy()
             p.oil_cx = self.p.oil_cx if cx is None else cx
             p.oil_cy = self.p.oil_cy if cy is None else cy
-        uz = torch.zeros(int(self.p.nz), dtype=torch.float64, device=self.device)
-        phi = torch.zeros_like(uz)
+        nz = int(self.p.nz)
+        prof = torch.empty(2 * nz, dtype=torch.float64, device=self.device)  # u_z, then phi: every z is written
         torch.cuda.synchronize(self.device)
-        check(lib().ssmd_centreline(ctypes.byref(p), ctypes.byref(self.fields), uz.data_ptr(),
-                                    phi.data_ptr(), self.stream))
-        self.sync()
-        return uz.cpu().numpy(), phi.cpu().numpy()
+        check(lib().ssmd_centreline(ctypes.byref(p), ctypes.byref(self.fields), prof.data_ptr(),
+                                    prof.data_ptr() + 8 * nz, self.stream))
+        with torch.cuda.stream(self.torch_stream):  # one read of both, in order after the kernel
+            host = prof.cpu().numpy()
+        return host[:nz].copy(), host[nz:].copy()
 
     _DROPLET = np.dtype([("root", "u4"), ("cells", "u4"), ("volume", "f8"), ("touches_inlet", "u4"), ("reserved", "u4")])
 
@@ -213,8 +214,7 @@ class Simulation:
         arr = np.zeros(k, dtype=[("root", "u4"), ("cells", "u4"), ("volume", "f8"), ("touches_inlet", "u4")])
         for name in arr.dtype.names:
             arr[name] = out[name][:k]
-        arr.sort(order="root")
-        return arr
+        return arr[np.argsort(arr["root"])]  # (roots are distinct)
 
     def check_status(self) -> int:
         v = ctypes.c_uint32()
