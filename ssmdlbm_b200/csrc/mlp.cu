@@ -31,11 +31,11 @@
 // dH2 = dR W3 and dZ2 = dH2 gelu'(z2 + b2) on the CUDA cores (N = 2 is too
 // narrow for an MMA), dH1 = dZ2 W2 on the tensor cores, dZ1 = dH1 gelu'(z1 +
 // b1); the weight and bias gradients (sums over a tile's 128 rows) on the
-// tensor cores too: the epilogues also write H1, H2, X, dZ1, dZ2 and dR
-// transposed (bf16, K = the tile's rows), and two MMAs per tile accumulate
-// dW2^T, dW3^T (G1) and dW1^T with the bias gradients (G2, through a row of
-// ones) in TMEM across the CTA's tiles; they run while the next tile's
-// features load.  The CTA's sums are then either added across CTAs with
+// tensor cores too: two MMAs per tile whose K is the tile's rows read the same
+// row-wise tiles X, H1, H2, dZ1, dZ2, dR as MN-major operands and accumulate
+// dW2^T, dW3^T (G1) and dW1^T with the bias gradients (G2, through a column of
+// ones in X) in TMEM across the CTA's tiles; they run while the next tile
+// begins.  The CTA's sums are then either added across CTAs with
 // atomics (ssmd_mlp_grad) or written as one row per CTA and summed in CTA
 // order by a second kernel (ssmd_mlp_grad_ws: the same bits on every run).  Every wait on an MMA is bounded: on timeout
 // the CTA records bit 0 of the status word, frees its TMEM and returns.
@@ -76,32 +76,33 @@ constexpr uint32_t col_z2() { return MODE == kTrain ? 64u : 0u; }
 template <int MODE>
 constexpr uint32_t col_r() { return MODE == kTrain ? 128u : 0u; }
 constexpr uint32_t cZ1 = 0, cDH1 = 192, cG1 = 256, cG2 = 336;
-constexpr int kGK = kRows;         // K of the weight-gradient MMAs: the tile's rows
-constexpr int kGB = 2 * kH + 16;   // rows of the gradient B tile: dZ1^T, dZ2^T, dR^T (2 of 16)
+constexpr int kGB = 2 * kH + 16;   // columns of the gradient tile: dZ1, dZ2, dR (2 of 16)
 constexpr uint64_t kMmaWaitNs = 1000000000ull;
 constexpr int kMaxGradCtas = 256; // rows of the deterministic gradient workspace
 
 // shared-memory map (bytes from an aligned base: 1024 bytes for training,
-// 128 for inference; the no-swizzle operand layout needs 16); training-only
-// tiles: W2^T, bf16 dZ2, and the operands of the weight-gradient MMAs, all
-// K-major with K = the tile's 128 rows:
-//   GA2 [16 x 128]: X^T (rows 0-11), a row of ones (12), zeros (13-15); the
-//       M = 128 MMA reads rows 16-127 from GA1 that follows (their products
-//       land in accumulator rows nobody reads)
-//   GA1 [128 x 128]: H1^T (rows 0-63), H2^T (rows 64-127)
-//   GB  [144 x 128]: dZ1^T (rows 0-63), dZ2^T (64-127), dR^T (128-129), zeros
-// so that G1 = GA1 GB[64..143]^T holds dW2^T and dW3^T, and G2 = GA2 GB^T
-// holds dW1^T and, in its ones row, the three bias gradients; then a small
-// scratch for the per-warp losses
-constexpr uint32_t sW2T = 49152, sDZ2 = 57344, sGA2 = 73728, sGA1 = sGA2 + 16 * kGK * 2,
-                   sGB = sGA1 + kRows * kGK * 2, sDY = sGB + kGB * kGK * 2;
-static_assert(sGA2 + (uint32_t)kRows * kGK * 2 <= sGB, "the M = 128 read of GA2 stays inside GA2 + GA1");
+// 128 for inference; the no-swizzle operand layout needs 16).  Training, all
+// bf16, 8 x 8 core matrices of 128 bytes, a row group of 8 rows after the other:
+//   X, twice [128 x 16]: columns 0-11 the features, 12 ones, 13-15 zero (this
+//       tile's and the next's: the gradient MMA reads the one while the other is written)
+//   HH [128 x 128]: H1 (columns 0-63), H2 (64-127)
+//   DZ [128 x 144]: dZ1 (0-63), dZ2 (64-127), dR (128-129), zeros
+// Each is a K-major operand (rows M) of the layers' MMAs and, with its rows as K, an
+// MN-major one of the gradient MMAs: G1 = HH^T DZ[:, 64..143] holds dW2^T and dW3^T, G2 =
+// X^T DZ holds dW1^T and, in its ones row, the three bias gradients (G2's M = 128
+// reads columns 16-127 past X: their products land in accumulator rows nobody
+// reads).  (Transposed copies of all six, 270 two-byte stores per row with
+// 4-way bank conflicts, were 4000 of the 14 000 cycles of a tile and 55 KB more.)
+constexpr uint32_t sXT = 0, kXBytes = kRows * kK1 * 2, sHH = 2 * kXBytes, sDZ = sHH + kRows * 2 * kH * 2,
+                   sW1T = sDZ + kRows * kGB * 2, sW3T = sW1T + kH * kK1 * 2, sW2T = sW3T + kN3 * kH * 2,
+                   sDY = sW2T + kH * kH * 2;
+constexpr uint32_t kXGroup = kK1 / 8 * 128, kHGroup = 2 * kH / 8 * 128, kDGroup = kGB / 8 * 128; // a row group's bytes
 template <int MODE>
 struct Layout {
     static constexpr bool T = MODE == kTrain;
     // inference: W1, W3, W2, then one activation tile that holds X, H1, H2 in turn
-    static constexpr uint32_t sW1 = T ? 4096 : 0, sW3 = T ? 6144 : 2048, sH1 = T ? 8192 : 12288,
-                              sW2 = T ? 24576 : 4096, sH2 = T ? 32768 : sH1, sX = T ? 0 : sH1;
+    static constexpr uint32_t sW1 = T ? sW1T : 0, sW3 = T ? sW3T : 2048, sH1 = 12288, sW2 = T ? sW2T : 4096, sH2 = sH1,
+                              sX = sH1;
     static constexpr uint32_t big = T ? sDY + kRows * kOut * 4 : sH1 + kRows * kH * 2;
     static constexpr uint32_t b1 = big, b2 = b1 + kH * 4, b3 = b2 + kH * 4, w3f = b3 + 16,
                               norm = w3f + (T ? kOut * kH * 4 : 0), bar = norm + 32 * 4, slot = bar + 8,
@@ -177,23 +178,23 @@ __device__ __forceinline__ void st8(unsigned char *tile, int r, int k0, int K, c
 
 
 // Copy a [ROWS x K] block of fp32 weights (row stride K), times `scale` (a
-// power of two), into a bf16 tile of ROWS_PAD rows (extra rows zero); TRANS:
-// element (r, k) = src[k * ROWS + r].  A thread converts 8 values of a row and
+// power of two), into a bf16 tile of ROWS_PAD rows (extra rows and the columns from KV on
+// zero).  A thread converts 8 values of a row and
 // stores them at once, and all its loads are in flight together: a CTA's
 // set-up is one round trip, not one per element of a thread (training kernel
-// on 65 536 rows, 4 tiles a CTA: 43 -> 40 us; forward of 1 M rows, 8 tiles a CTA: 75 ->
+// on 65 536 rows, 4 tiles a CTA: 3 us of 43; forward of 1 M rows, 8 tiles a CTA: 75 ->
 // 67; refresh of 96 x 96 x 384 cells: 238 -> 229).
-template <int ROWS, int ROWS_PAD, int K, bool TRANS, int THREADS>
+template <int ROWS, int ROWS_PAD, int K, int THREADS, int KV = K>
 __device__ __forceinline__ void load_weights(unsigned char *tile, const float *src, int tid, float scale = 1.0f) {
     constexpr int CHUNKS = ROWS_PAD * (K / 8);
 #pragma unroll
     for (int c0 = 0; c0 < CHUNKS; c0 += THREADS) {
         const int c = c0 + tid;
         if (CHUNKS % THREADS != 0 && c >= CHUNKS) break;
-        const int r = TRANS ? c % ROWS_PAD : c / (K / 8), k0 = 8 * (TRANS ? c / ROWS_PAD : c % (K / 8));
+        const int r = c / (K / 8), k0 = 8 * (c % (K / 8));
         float v[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = r < ROWS ? __ldg(src + (TRANS ? (k0 + i) * ROWS + r : r * K + k0 + i)) * scale : 0.f;
+        for (int i = 0; i < 8; ++i) v[i] = r < ROWS && k0 + i < KV ? __ldg(src + r * K + k0 + i) * scale : 0.f;
         st8(tile, r, k0, K, v);
     }
 }
@@ -207,22 +208,13 @@ __device__ __forceinline__ bool wait_mma(uint64_t *bar, uint32_t phase, volatile
     return ok;
 }
 
-// Element (m, k) of a K-major bf16 tile with K = kGK (the weight-gradient
-// operands: the tile's rows r are their K).
-__device__ __forceinline__ void st_g(unsigned char *tile, int m, int k, uint16_t bits) {
-    *reinterpret_cast<uint16_t *>(tile + umma::kmajor_offset(m, k, kGK)) = bits;
-}
-__device__ __forceinline__ uint16_t bf16_bits(float v) {
-    const __nv_bfloat16 h = __float2bfloat16_rn(v);
-    return *reinterpret_cast<const uint16_t *>(&h);
-}
-
 // Bias + GELU of 16 accumulator columns v (columns c0 .. c0 + 15 of the layer)
-// into row r of a [128 x 64] bf16 tile (TWICE: 2 gelu, for a next layer staged
-// with halved weights); pk returns the bf16 pairs.
-template <bool TWICE>
+// into columns t0 .. t0 + 15 of row r of a bf16 tile of K columns (TWICE: 2 gelu, for a
+// next layer staged with halved weights).
+template <bool TWICE, int K>
 __device__ __forceinline__ void gelu16(const float (&v)[16], const float *bias, int c0, unsigned char *tile, int r,
-                                       uint32_t (&pk)[8]) {
+                                       int t0) {
+    uint32_t pk[8];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const float4 b = *reinterpret_cast<const float4 *>(bias + c0 + 4 * i);
@@ -231,8 +223,8 @@ __device__ __forceinline__ void gelu16(const float (&v)[16], const float *bias, 
         pk[2 * i] = pack2(g0.x, g0.y);
         pk[2 * i + 1] = pack2(g1.x, g1.y);
     }
-    *reinterpret_cast<uint4 *>(tile + umma::kmajor_offset(r, c0, kH)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-    *reinterpret_cast<uint4 *>(tile + umma::kmajor_offset(r, c0 + 8, kH)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+    *reinterpret_cast<uint4 *>(tile + umma::kmajor_offset(r, t0, K)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+    *reinterpret_cast<uint4 *>(tile + umma::kmajor_offset(r, t0 + 8, K)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
 }
 
 // Inference epilogue of a 64-column accumulator: the TMEM load of columns
@@ -247,24 +239,16 @@ __device__ __forceinline__ void hidden_epilogue(uint32_t taddr, const float *bia
 #pragma unroll
         for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(nxt[i]);
         if (c < 3) umma::tmem_ld16_issue(taddr + 16 * (c + 1), nxt);
-        uint32_t pk[8];
-        gelu16<true>(v, bias, 16 * c, tile, r, pk);
+        gelu16<true, kH>(v, bias, 16 * c, tile, r, 16 * c);
     }
 }
 
-// Training epilogue of columns 16 grp .. 16 grp + 15: the same bf16 values also
-// into column r, rows trow0 + 16 grp .., of a weight-gradient operand tile.
-__device__ __forceinline__ void hidden_epilogue16(uint32_t taddr, const float *bias, unsigned char *tile, int r, int grp,
-                                                  unsigned char *ttile, int trow0) {
+// Training epilogue of columns 16 grp .. 16 grp + 15, into HH from column t0 on.
+__device__ __forceinline__ void hidden_epilogue16(uint32_t taddr, const float *bias, unsigned char *hh, int r, int grp,
+                                                  int t0) {
     float v[16];
     umma::tmem_ld16(taddr + 16 * grp, v);
-    uint32_t pk[8];
-    gelu16<false>(v, bias, 16 * grp, tile, r, pk);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        st_g(ttile, trow0 + 16 * grp + 2 * i, r, (uint16_t)(pk[i] & 0xFFFFu));
-        st_g(ttile, trow0 + 16 * grp + 2 * i + 1, r, (uint16_t)(pk[i] >> 16));
-    }
+    gelu16<false, 2 * kH>(v, bias, 16 * grp, hh, r, t0 + 16 * grp);
 }
 
 // The 12 standardised features of one row into x[16] (columns 12-15 zero);
@@ -324,9 +308,9 @@ __global__ void __launch_bounds__(kThreadsMlp, 7) mlp_kernel(const MlpArgs a) {
         fence_barrier_init();
     }
     // W2 and W3 are fed with 2 gelu(z): halved weights, the same products
-    load_weights<kH, kH, kK1, false, kThreadsMlp>(sm + L::sW1, net + oW1, tid);
-    load_weights<kH, kH, kH, false, kThreadsMlp>(sm + L::sW2, net + oW2, tid, 0.5f);
-    load_weights<kOut, kN3, kH, false, kThreadsMlp>(sm + L::sW3, net + oW3, tid, 0.5f);
+    load_weights<kH, kH, kK1, kThreadsMlp>(sm + L::sW1, net + oW1, tid);
+    load_weights<kH, kH, kH, kThreadsMlp>(sm + L::sW2, net + oW2, tid, 0.5f);
+    load_weights<kOut, kN3, kH, kThreadsMlp>(sm + L::sW3, net + oW3, tid, 0.5f);
     for (int e = tid; e < kH; e += kThreadsMlp) {
         b1[e] = net[oB1 + e];
         b2[e] = net[oB2 + e];
@@ -446,7 +430,8 @@ struct TrainRow {
 // kernel is a chain of MMA round trips and epilogues per tile; with one thread
 // per row (4 warps per SM, one per scheduler) the epilogues' ~5000 instructions
 // ran at the latency of one warp: 15 us a tile, 62 us for 65 536 rows; with four
-// threads per row 40, the gather included.  The rows of a mini-batch are read through their
+// threads per row 40, the gather included, and 28 with the gradient MMAs reading row-wise
+// tiles (see the shared-memory map) and a row's index loaded a tile ahead of the row.  The rows of a mini-batch are read through their
 // indices (a.rows), the next tile's while this one's layers run: gathering them first took
 // three launches and 50 us of the 128 us step.  Every value and every sum is in
 // the order of one thread per row: the same bits.
@@ -497,7 +482,9 @@ __global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpAr
         d.w1 = a.weight ? a.weight[s * kOut + 1] : 1.0f;
         return d;
     };
+    // (a row's index is loaded a tile before the row itself: two round trips, neither waited for)
     TrainRow cur = fetch((int64_t)blockIdx.x < tiles ? source(blockIdx.x) : -1);
+    int64_t nsrc = (int64_t)blockIdx.x + gridDim.x < tiles ? source((int64_t)blockIdx.x + gridDim.x) : -1;
 
     // ---- set-up: TMEM, barrier, weights
     if (warp == 0) umma::tmem_alloc(slot, tmem_cols<kTrain>());
@@ -506,10 +493,9 @@ __global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpAr
         *abort_flag = 0u;
         fence_barrier_init();
     }
-    load_weights<kH, kH, kK1, false, kThreadsTrain>(sm + L::sW1, net + oW1, tid);
-    load_weights<kH, kH, kH, false, kThreadsTrain>(sm + L::sW2, net + oW2, tid);
-    load_weights<kOut, kN3, kH, false, kThreadsTrain>(sm + L::sW3, net + oW3, tid);
-    load_weights<kH, kH, kH, true, kThreadsTrain>(sm + sW2T, net + oW2, tid); // (i, o) = W2[o][i]
+    load_weights<kH, kH, kK1, kThreadsTrain, kIn>(sm + L::sW1, net + oW1, tid); // (X's column 12 is the gradients' ones)
+    load_weights<kH, kH, kH, kThreadsTrain>(sm + L::sW2, net + oW2, tid);
+    load_weights<kOut, kN3, kH, kThreadsTrain>(sm + L::sW3, net + oW3, tid);
     if (tid < kH) {
         b1[tid] = net[oB1 + tid];
         b2[tid] = net[oB2 + tid];
@@ -517,67 +503,53 @@ __global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpAr
     if (tid < kOut * kH) w3f[tid] = net[oW3 + tid];
     if (tid < kOut) b3[tid] = net[oB3 + tid];
     if (tid < kNet - kParams) norm[tid] = net[kParams + tid];
-    if (grp == 0) {
-        // the rows of the gradient operands that no tile writes: GA2 row 12
-        // all ones (its products are the column sums, the bias gradients),
-        // rows 13-15 and GB rows 130-143 zero
-        const uint16_t one = bf16_bits(1.0f);
-        st_g(sm + sGA2, 12, r, one);
-        for (int m = 13; m < 16; ++m) st_g(sm + sGA2, m, r, 0);
-        for (int m = 2 * kH + kOut; m < kGB; ++m) st_g(sm + sGB, m, r, 0);
+    if (grp == 0) { // the columns of DZ that no tile writes: 130-143 (128-129 with every tile)
+        *reinterpret_cast<uint4 *>(sm + sDZ + umma::kmajor_offset(r, 2 * kH, kGB)) = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4 *>(sm + sDZ + umma::kmajor_offset(r, 2 * kH + 8, kGB)) = make_uint4(0u, 0u, 0u, 0u);
     }
     __syncthreads();
 
     const uint32_t sbase = smem_addr(sm);
     uint32_t phase = 0;
     bool ok = true;
-    // the weight-gradient MMAs of a tile run while the next tile begins; gpend
-    // says they are in flight (waited for before the next tile writes their
-    // operands, and after the last tile)
-    bool gpend = false, gfirst = true;
+    // the weight-gradient MMAs of a tile run while the next tile begins: the commit
+    // of that tile's first MMA covers them, before anything they read is written
+    bool gfirst = true;
+    uint32_t xbuf = 0;
     float lsum = 0.f;
     const uint32_t tmem = *slot;
     const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
 
     for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-        const int64_t next = tile + gridDim.x;
-        const int64_t nsrc = next < tiles ? source(next) : -1;
+        const uint32_t sX = sXT + xbuf * kXBytes;
         {
-            // group 3 writes the zero padding of X (columns 12-15)
+            // group 3 writes columns 12-15: one, zeros
             float x[4];
             const float f[4] = {cur.f.x, cur.f.y, cur.f.z, cur.f.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-                x[i] = cur.valid && grp < kIn / 4 ? (f[i] - norm[4 * grp + i]) * norm[kIn + 4 * grp + i] : 0.f;
-            *reinterpret_cast<uint2 *>(sm + L::sX + umma::kmajor_offset(r, 4 * grp, kK1)) =
+                x[i] = grp == kIn / 4 ? (i == 0 ? 1.0f : 0.f)
+                                      : (cur.valid ? (f[i] - norm[4 * grp + i]) * norm[kIn + 4 * grp + i] : 0.f);
+            *reinterpret_cast<uint2 *>(sm + sX + umma::kmajor_offset(r, 4 * grp, kK1)) =
                 make_uint2(pack2(x[0], x[1]), pack2(x[2], x[3]));
-            if (gpend) { // the previous tile's gradient MMAs read GA2, GA1, GB
-                ok = wait_mma(bar, phase, abort_flag);
-                phase ^= 1u;
-                gpend = false;
-                if (!ok) break;
-            }
-            if (grp < kIn / 4) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) st_g(sm + sGA2, 4 * grp + i, r, bf16_bits(x[i])); // X^T
-            }
         }
         fence_proxy_async(); // generic-proxy smem writes -> visible to the tensor core
         umma::fence_before_sync();
-        __syncthreads(); // also: every TMEM read and MMA of the previous tile is complete
+        __syncthreads(); // also: every TMEM read of the previous tile is complete
 
         // ---- layer 1
         if (tid == 0) {
             umma::fence_after_sync();
-            umma::mma_bf16(tmem + cZ1, umma::smem_desc(sbase + L::sX, 128, 256),
+            umma::mma_bf16(tmem + cZ1, umma::smem_desc(sbase + sX, 128, kXGroup),
                            umma::smem_desc(sbase + L::sW1, 128, 256), umma::idesc_bf16(128, kH), false);
             umma::commit(bar);
         }
         const TrainRow nxt = fetch(nsrc);
+        nsrc = tile + 2 * (int64_t)gridDim.x < tiles ? source(tile + 2 * (int64_t)gridDim.x) : -1;
         ok = wait_mma(bar, phase, abort_flag);
         phase ^= 1u;
         if (!ok) break;
-        hidden_epilogue16(lane_base + cZ1, b1, sm + L::sH1, r, grp, sm + sGA1, 0); // (H1^T)
+        hidden_epilogue16(lane_base + cZ1, b1, sm + sHH, r, grp, 0);
         fence_proxy_async();
         umma::fence_before_sync();
         __syncthreads();
@@ -586,7 +558,7 @@ __global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpAr
         if (tid == 0) {
             umma::fence_after_sync();
             for (int ks = 0; ks < kH / 16; ++ks)
-                umma::mma_bf16(tmem + col_z2<kTrain>(), umma::smem_desc(sbase + L::sH1 + 256 * ks, 128, 1024),
+                umma::mma_bf16(tmem + col_z2<kTrain>(), umma::smem_desc(sbase + sHH + 256 * ks, 128, kHGroup),
                                umma::smem_desc(sbase + L::sW2 + 256 * ks, 128, 1024), umma::idesc_bf16(128, kH),
                                ks > 0);
             umma::commit(bar);
@@ -594,7 +566,7 @@ __global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpAr
         ok = wait_mma(bar, phase, abort_flag);
         phase ^= 1u;
         if (!ok) break;
-        hidden_epilogue16(lane_base + col_z2<kTrain>(), b2, sm + L::sH2, r, grp, sm + sGA1, kH); // (H2^T)
+        hidden_epilogue16(lane_base + col_z2<kTrain>(), b2, sm + sHH, r, grp, kH);
         fence_proxy_async();
         umma::fence_before_sync();
         __syncthreads();
@@ -603,7 +575,7 @@ __global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpAr
         if (tid == 0) {
             umma::fence_after_sync();
             for (int ks = 0; ks < kH / 16; ++ks)
-                umma::mma_bf16(tmem + col_r<kTrain>(), umma::smem_desc(sbase + L::sH2 + 256 * ks, 128, 1024),
+                umma::mma_bf16(tmem + col_r<kTrain>(), umma::smem_desc(sbase + sHH + kH / 8 * 128 + 256 * ks, 128, kHGroup),
                                umma::smem_desc(sbase + L::sW3 + 256 * ks, 128, 1024), umma::idesc_bf16(128, kN3),
                                ks > 0);
             umma::commit(bar);
@@ -629,10 +601,7 @@ __global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpAr
             d0 = 2.0f * cur.w0 * e0 * inv_n;
             d1 = 2.0f * cur.w1 * e1 * inv_n;
         }
-        if (grp == 0) {
-            st_g(sm + sGB, 2 * kH + 0, r, bf16_bits(d0)); // dR^T
-            st_g(sm + sGB, 2 * kH + 1, r, bf16_bits(d1));
-        }
+        if (grp == 0) *reinterpret_cast<uint32_t *>(sm + sDZ + umma::kmajor_offset(r, 2 * kH, kGB)) = pack2(d0, d1); // dR
         // ---- dZ2 = (dR W3) * gelu'(z2 + b2)
         {
             float v[16];
@@ -642,21 +611,20 @@ __global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpAr
                 const int j = 16 * grp + i;
                 const float dh = fmaf(d0, w3f[j], d1 * w3f[kH + j]);
                 v[i] = dh * gelu_grad(v[i] + b2[j]);
-                st_g(sm + sGB, kH + j, r, bf16_bits(v[i])); // dZ2^T
             }
-            st8(sm + sDZ2, r, 16 * grp, kH, v);
-            st8(sm + sDZ2, r, 16 * grp + 8, kH, v + 8);
+            st8(sm + sDZ, r, kH + 16 * grp, kGB, v);
+            st8(sm + sDZ, r, kH + 16 * grp + 8, kGB, v + 8);
         }
         fence_proxy_async();
         umma::fence_before_sync();
         __syncthreads();
-        // ---- dH1 = dZ2 W2 (B = W2^T, K-major)
+        // ---- dH1 = dZ2 W2 (B: W2 with its outputs o as K, MN-major)
         if (tid == 0) {
             umma::fence_after_sync();
             for (int ks = 0; ks < kH / 16; ++ks)
-                umma::mma_bf16(tmem + cDH1, umma::smem_desc(sbase + sDZ2 + 256 * ks, 128, 1024),
-                               umma::smem_desc(sbase + sW2T + 256 * ks, 128, 1024), umma::idesc_bf16(128, kH),
-                               ks > 0);
+                umma::mma_bf16(tmem + cDH1, umma::smem_desc(sbase + sDZ + kH / 8 * 128 + 256 * ks, 128, kDGroup),
+                               umma::smem_desc(sbase + L::sW2 + 2048 * ks, 1024, 128),
+                               umma::idesc_bf16(128, kH, false, true), ks > 0);
             umma::commit(bar);
         }
         ok = wait_mma(bar, phase, abort_flag);
@@ -667,37 +635,35 @@ __global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpAr
             umma::tmem_ld16(lane_base + cDH1 + 16 * grp, dh);
             umma::tmem_ld16(lane_base + cZ1 + 16 * grp, z);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int j = 16 * grp + i;
-                st_g(sm + sGB, j, r, bf16_bits(dh[i] * gelu_grad(z[i] + b1[j]))); // dZ1^T
-            }
+            for (int i = 0; i < 16; ++i) dh[i] *= gelu_grad(z[i] + b1[16 * grp + i]);
+            st8(sm + sDZ, r, 16 * grp, kGB, dh); // dZ1
+            st8(sm + sDZ, r, 16 * grp + 8, kGB, dh + 8);
         }
         fence_proxy_async();
         umma::fence_before_sync();
         __syncthreads();
         // ---- weight and bias gradients of this tile, summed over its 128
         // rows (the MMAs' K) into the CTA's accumulators G1 and G2:
-        //   G1 [128 x 80]  += GA1 GB[64..143]^T: rows 0-63 dW2^T, rows 64-127 cols 64-65 dW3^T
-        //   G2 [128 x 144] += GA2 GB^T: rows 0-11 cols 0-63 dW1^T; row 12: db1, db2, db3
+        //   G1 [128 x 80]  += HH^T DZ[:, 64..143]: rows 0-63 dW2^T, rows 64-127 cols 64-65 dW3^T
+        //   G2 [128 x 144] += X^T DZ: rows 0-11 cols 0-63 dW1^T; row 12: db1, db2, db3
         if (tid == 0) {
             umma::fence_after_sync();
-            for (int ks = 0; ks < kGK / 16; ++ks)
-                umma::mma_bf16(tmem + cG1, umma::smem_desc(sbase + sGA1 + 256 * ks, 128, 2048),
-                               umma::smem_desc(sbase + sGB + (kH / 8) * 2048 + 256 * ks, 128, 2048),
-                               umma::idesc_bf16(128, kGB - kH), !gfirst || ks > 0);
-            for (int ks = 0; ks < kGK / 16; ++ks)
-                umma::mma_bf16(tmem + cG2, umma::smem_desc(sbase + sGA2 + 256 * ks, 128, 2048),
-                               umma::smem_desc(sbase + sGB + 256 * ks, 128, 2048), umma::idesc_bf16(128, kGB),
-                               !gfirst || ks > 0);
-            umma::commit(bar);
+            for (int ks = 0; ks < kRows / 16; ++ks)
+                umma::mma_bf16(tmem + cG1, umma::smem_desc(sbase + sHH + 2 * kHGroup * ks, kHGroup, 128),
+                               umma::smem_desc(sbase + sDZ + kH / 8 * 128 + 2 * kDGroup * ks, kDGroup, 128),
+                               umma::idesc_bf16(128, kGB - kH, true, true), !gfirst || ks > 0);
+            for (int ks = 0; ks < kRows / 16; ++ks)
+                umma::mma_bf16(tmem + cG2, umma::smem_desc(sbase + sX + 2 * kXGroup * ks, kXGroup, 128),
+                               umma::smem_desc(sbase + sDZ + 2 * kDGroup * ks, kDGroup, 128),
+                               umma::idesc_bf16(128, kGB, true, true), !gfirst || ks > 0);
         }
-        gpend = true;
+        xbuf ^= 1u;
         gfirst = false;
         cur = nxt;
     }
-    if (ok && gpend) {
+    if (ok && !gfirst) {
+        if (tid == 0) umma::commit(bar); // the last tile's gradient MMAs
         ok = wait_mma(bar, phase, abort_flag);
-        phase ^= 1u;
     }
 
     if (ok) {
@@ -722,17 +688,26 @@ __global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpAr
                 put(oW3 + 1 * kH + (m - kH), v[1]);
             }
             if ((warp & 3) == 0) { // warp-collective loads: lanes 0-11 dW1, lane 12 the biases
-                for (int c = grp; c < kGB / 16; c += kTrainGroups) {
-                    umma::tmem_ld16(lane_base + cG2 + 16 * c, v);
+                umma::tmem_ld16(lane_base + cG2 + 16 * grp, v);
+                if (m < kK1) {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const int col = 16 * c + i;
-                        if (col < kH && m < kK1) put(oW1 + col * kK1 + m, m < kIn ? v[i] : 0.f); // dW1[o][m]
-                        if (m == kIn) {
-                            if (col < kH) put(oB1 + col, v[i]);
-                            else if (col < 2 * kH) put(oB2 + col - kH, v[i]);
-                            else if (col < 2 * kH + kOut) put(oB3 + col - 2 * kH, v[i]);
-                        }
+                    for (int i = 0; i < 16; ++i) put(oW1 + (16 * grp + i) * kK1 + m, m < kIn ? v[i] : 0.f); // dW1[o][m]
+                }
+                if (m == kIn) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) put(oB1 + 16 * grp + i, v[i]);
+                }
+                umma::tmem_ld16(lane_base + cG2 + kH + 16 * grp, v);
+                if (m == kIn) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) put(oB2 + 16 * grp + i, v[i]);
+                }
+                if (grp == 0) {
+                    float w[2];
+                    umma::tmem_ld2(lane_base + cG2 + 2 * kH, w);
+                    if (m == kIn) {
+                        put(oB3 + 0, w[0]);
+                        put(oB3 + 1, w[1]);
                     }
                 }
             }

@@ -6,7 +6,11 @@
 // matrices adjacent along K are LBO = 128 bytes apart, core matrices adjacent
 // along M (or N) are SBO = (K / 8) * 128 bytes apart.  One MMA of kind::f16
 // consumes K = 16, i.e. two core matrices along K, so the k-th K step of a
-// wider tile starts 256 k bytes after its base.  The accumulator of an
+// wider tile starts 256 k bytes after its base.  The same bytes are an MN-major
+// operand whose K is the tile's rows and whose M (or N) its columns: a core matrix
+// holds 8 K rows of 8 contiguous M values, core matrices adjacent along K are LBO
+// = (columns / 8) * 128 bytes apart, along M SBO = 128, and the k-th K step starts
+// 2 LBO k bytes after the base.  The accumulator of an
 // M = 128 MMA occupies TMEM lanes 0..127 (row i -> lane i) and N consecutive
 // 32-bit columns; warp w of the CTA may read lanes 32 w .. 32 w + 31.
 #pragma once
@@ -35,10 +39,11 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
     return d;
 }
 
-// Instruction descriptor of kind::f16: FP32 accumulator, bf16 A and B, both
-// K-major, shape M x N.
-__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+// Instruction descriptor of kind::f16: FP32 accumulator, bf16 A and B, shape
+// M x N, each operand K-major or (mn_a, mn_b) MN-major.
+__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, bool mn_a = false, bool mn_b = false) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)mn_a << 15) | ((uint32_t)mn_b << 16) |
+           ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
 // D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
