@@ -387,13 +387,7 @@ int launch_step(const ssmd_params &p, const LBMFields &fl, uint64_t step, uint32
     const Geometry &G = a.geo;
     auto faces = [&](auto kind, uint32_t n0, uint32_t n1) {
         constexpr int K = decltype(kind)::value;
-        const dim3 grid = face_grid<Q, K>(n0, n1), block(kFaceX, kFaceY);
-        if constexpr (Q == 27 && sizeof(T) == 4 && kFaces<K> == 2)
-            if (one_thread_per_cell(grid, sms)) {
-                bc_cell_kernel<Q, T, TG, K><<<dim3(grid.x / (kFaces<K> * kSlots<Q, K>), grid.y, kFaces<K>), block, 0, st>>>(a);
-                return;
-            }
-        bc_kernel<Q, T, TG, K><<<grid, block, 0, st>>>(a);
+        bc_kernel<Q, T, TG, K><<<face_grid<Q, K>(n0, n1), dim3(kFaceX, kFaceY), 0, st>>>(a);
     };
     if (G.bcy == BC_JET) faces(ic<BK_JET_Y>{}, G.nx, G.nz);
     if (G.bcz == BC_JET) faces(ic<BK_JET_Z>{}, G.nx, G.ny);

@@ -339,8 +339,7 @@ constexpr int kSlots = K == BK_JET_Y || K == BK_JET_Z ? kFaceDirs<Q> + 1 : 2 * k
 // lattices: blocks of kFaceX x kFaceY face cells, blockIdx.x the tiles along the
 // first axis times the slots of the faces.  (Several slots per thread in a loop, so
 // that all blocks of a large face are resident at once, lost to the round trips
-// that then follow one another: 256 x 256 face 5.6 -> 7.4 us, crossflow 21 -> 26; the
-// one case where it wins is bc_cell_kernel's.)
+// that then follow one another: 256 x 256 face 5.6 -> 7.4 us, crossflow 21 -> 26.)
 template <int Q, int K>
 inline dim3 face_grid(uint32_t n0, uint32_t n1, unsigned count = 1) {
     return dim3((n0 + kFaceX - 1) / kFaceX * (kFaces<K> * kSlots<Q, K>), (n1 + kFaceY - 1) / kFaceY, count);
@@ -366,33 +365,6 @@ __device__ __forceinline__ void bc_face(const StepArgs<TF, TG> &a) {
         if (G.bcx == BC_COPY) bc_copy_x_at<Q>(a, i0, i1, s);
     } else {
         if (G.bcy == BC_COPY) bc_copy_y_at<Q>(a, i0, i1, s);
-    }
-}
-
-// Large jet faces of D3Q27 FP32: a thread takes all slots of its cell, one after
-// another.  The split pays while its blocks are resident at once (16 of 128 threads on
-// an SM).  Above that later blocks wait for a place, and where other lattices' kernels
-// fill the device those places come slowly.  128 x 128 x 512 jet, three lattices on
-// their own streams, us a pass of ten steps: 4875 split, 4845 so; one lattice alone 5009
-// and 5015.  Not for 16-bit storage (3815 to 3773, but alone 4115 to 4205) nor
-// for D3Q19 (256 x 256 x 256 6256 to 6290).
-inline bool one_thread_per_cell(const dim3 &split, int sms) {
-    return (long)split.x * split.y > 2048 / (kFaceX * kFaceY) * (long)sms;
-}
-template <int Q, class TF, class TG, int K>
-__global__ void __launch_bounds__(kFaceX * kFaceY) bc_cell_kernel(const StepArgs<TF, TG> a) {
-    static_assert(K == BK_JET_Y || K == BK_JET_Z, "jet faces");
-    const bool in = blockIdx.z == 0;
-    const int i0 = (int)(blockIdx.x * kFaceX + threadIdx.x), i1 = (int)(blockIdx.y * kFaceY + threadIdx.y);
-#pragma unroll 1
-    for (int k = 0; k < kSlots<Q, K>; ++k) {
-        if constexpr (K == BK_JET_Y) {
-            if (in) bc_water_inflow_at<Q>(a, i0, i1, k);
-            else bc_outflow_y_at<Q>(a, i0, i1, k);
-        } else {
-            if (in) bc_oil_inflow_at<Q>(a, i0, i1, k);
-            else bc_outflow_z_at<Q>(a, i0, i1, k);
-        }
     }
 }
 

@@ -65,19 +65,3 @@ def test_periodic_xy_instantiation_gives_the_same_bits(shape, box, vs, storage):
         assert sim.check_status() == 0
     for k in got[0]:
         assert np.array_equal(got[0][k], got[1][k]), k
-
-
-@pytest.mark.parametrize("faces", [(COPY, JET, JET), (PER, JET, JET), (PER, PER, JET)])
-@pytest.mark.parametrize("shape", [(130, 9, 121), (129, 122, 7), (96, 157, 6), (96, 160, 6)],
-                         ids=["large y face", "large z face", "just split", "just not split"])
-def test_large_jet_faces_match_oracle(shape, faces):
-    """FP32 D3Q27 jet faces of more tiles than are resident at once: one thread per cell."""
-    from ssmdlbm_b200.lbm import Simulation
-    p = _params(shape, faces, 27)
-    sim, o = Simulation(p), Oracle(p, 32)
-    m = seeded_macros((p.nz, p.ny, p.nx), seed=11)
-    sim.init_from_macros(*m)
-    o.init_macros(*m)
-    sim.step(1, store_macros=True)
-    o.step(1)
-    compare_fields(sim_fields(sim), oracle_fields(o), 5e-6)
