@@ -339,7 +339,11 @@ constexpr int kSlots = K == BK_JET_Y || K == BK_JET_Z ? kFaceDirs<Q> + 1 : 2 * k
 // lattices: blocks of kFaceX x kFaceY face cells, blockIdx.x the tiles along the
 // first axis times the slots of the faces.  (Several slots per thread in a loop, so
 // that all blocks of a large face are resident at once, lost to the round trips
-// that then follow one another: 256 x 256 face 5.6 -> 7.4 us, crossflow 21 -> 26.)
+// that then follow one another: 256 x 256 face 5.6 -> 7.4 us, crossflow 21 -> 26.  The one
+// loss: three 128 x 128 x 512 D3Q27 FP32 jets on streams of their own, whose bulk blocks
+// fill every SM, take 484 us for each step instead of 480; one alone in a replayed graph
+// takes 450 instead of 456.  One thread per cell there brought the 484 to 481 and the 450
+// to 459.)
 template <int Q, int K>
 inline dim3 face_grid(uint32_t n0, uint32_t n1, unsigned count = 1) {
     return dim3((n0 + kFaceX - 1) / kFaceX * (kFaces<K> * kSlots<Q, K>), (n1 + kFaceY - 1) / kFaceY, count);
