@@ -43,37 +43,60 @@ __device__ __forceinline__ Dir direction(int q) {
     return d;
 }
 
-// Shifted equilibrium of direction c (D3Q19.cuh:133-140, D3Q27.cuh:147-154).
-template <int Q>
-__device__ __forceinline__ float feq_of(float cx, float cy, float cz, float w, float rho, float ux, float uy,
-                                        float uz) {
-    const float uu = 1.5f * (ux * ux + uy * uy + uz * uz);
-    const float cu = 3.0f * (cx * ux + cy * uy + cz * uz);
-    float b = 1.0f - uu + cu + 0.5f * cu * cu;
-    if constexpr (Q == 27) b += cu * cu * cu * float(1.0 / 6.0) - uu * cu;
-    return w * rho * b - w;
-}
-template <int Q, int q>
-__device__ __forceinline__ float feq_dir(float rho, float ux, float uy, float uz) {
-    return feq_of<Q>(float(cx27(q)), float(cy27(q)), float(cz27(q)), VS<Q>::w(q), rho, ux, uy, uz);
+// The boundary values' arithmetic is written out, one rounding per operation: a
+// `a * b + c` left to the compiler is fused in an order that depends on what is
+// constant around it, and a last bit at the inlet grows in the liquid column.  Which
+// product of a sum of two enters fused (the other one is rounded first) is
+// therefore a rule on the direction: these are the bits of direction-by-direction code
+// with constant c.
+__device__ __forceinline__ float two_products(float a, float x, float b, float y, bool second_fused) {
+    return fmaf(second_fused ? b : a, second_fused ? y : x,
+                __fmul_rn(second_fused ? a : b, second_fused ? x : y));
 }
 
-// Hermite non-equilibrium of direction c (D3Q19.cuh:142-161, D3Q27.cuh:156-185).
+// Shifted equilibrium of direction d (D3Q19.cuh:133-140, D3Q27.cuh:147-154).
 template <int Q>
-__device__ __forceinline__ float fneq_of(float cx, float cy, float cz, float w, float pxx, float pyy, float pzz,
-                                         float pxy, float pxz, float pyz, float ux, float uy, float uz) {
-    float h = (cx * cx - kCs2) * pxx + (cy * cy - kCs2) * pyy + (cz * cz - kCs2) * pzz +
-              2.0f * (cx * cy * pxy + cx * cz * pxz + cy * cz * pyz);
+__device__ __forceinline__ float feq_of(const Dir &d, float rho, float ux, float uy, float uz) {
+    const float u2 = fmaf(uz, uz, fmaf(ux, ux, __fmul_rn(uy, uy)));
+    const float uu = __fmul_rn(1.5f, u2);
+    const float cu = __fmul_rn(3.0f, fmaf(d.cz, uz, fmaf(d.cx, ux, __fmul_rn(d.cy, uy))));
+    float b = Q == 27 ? __fsub_rn(1.0f, uu) : fmaf(-1.5f, u2, 1.0f);
+    b = fmaf(__fmul_rn(0.5f, cu), cu, __fadd_rn(b, cu));
     if constexpr (Q == 27) {
-        h += 3.0f * ((cx * cx * cy - kCs2 * cy) * (pxx * uy + 2.0f * ux * pxy) +
-                     (cx * cx * cz - kCs2 * cz) * (pxx * uz + 2.0f * ux * pxz) +
-                     (cx * cy * cy - kCs2 * cx) * (pyy * ux + 2.0f * uy * pxy) +
-                     (cy * cy * cz - kCs2 * cz) * (pyy * uz + 2.0f * uy * pyz) +
-                     (cx * cz * cz - kCs2 * cx) * (pzz * ux + 2.0f * uz * pxz) +
-                     (cy * cz * cz - kCs2 * cy) * (pzz * uy + 2.0f * uz * pyz)) +
-             6.0f * (cx * cy * cz) * (ux * pyz + uy * pxz + uz * pxy);
+        const float cu3 = __fmul_rn(__fmul_rn(cu, cu), cu);
+        b = __fadd_rn(b, fmaf(cu3, float(1.0 / 6.0), -__fmul_rn(uu, cu)));
     }
-    return (w * 4.5f) * h;
+    return fmaf(__fmul_rn(d.w, rho), b, -d.w);
+}
+
+template <int Q, int q>
+__device__ __forceinline__ float feq_dir(float rho, float ux, float uy, float uz) {
+    constexpr Dir d{float(cx27(q)), float(cy27(q)), float(cz27(q)), VS<Q>::w(q), cx27(q), cy27(q), cz27(q)};
+    return feq_of<Q>(d, rho, ux, uy, uz);
+}
+
+// Hermite non-equilibrium of direction d (D3Q19.cuh:142-161, D3Q27.cuh:156-185).
+template <int Q>
+__device__ __forceinline__ float fneq_of(const Dir &d, float pxx, float pyy, float pzz, float pxy, float pxz,
+                                         float pyz, float ux, float uy, float uz) {
+    const float cx = d.cx, cy = d.cy, cz = d.cz; // -1, 0, 1: products with them are exact
+    const float kx = cx * cx - kCs2, ky = cy * cy - kCs2, kz = cz * cz - kCs2;
+    float h = fmaf(kz, pzz, two_products(kx, pxx, ky, pyy, d.ix == 0 && d.iy != 0));
+    h = fmaf(2.0f, fmaf(cy * cz, pyz, fmaf(cx * cz, pxz, __fmul_rn(cx * cy, pxy))), h);
+    if constexpr (Q == 27) {
+        const float ux2 = 2.0f * ux, uy2 = 2.0f * uy, uz2 = 2.0f * uz;
+        const float c0 = kx * cy, c1 = kx * cz;
+        float s = two_products(c0, fmaf(ux2, pxy, __fmul_rn(pxx, uy)), c1, fmaf(ux2, pxz, __fmul_rn(pxx, uz)),
+                               c0 < 0.0f && c1 > 0.0f);
+        s = fmaf(ky * cx, fmaf(pyy, ux, __fmul_rn(uy2, pxy)), s);
+        s = fmaf(ky * cz, fmaf(uy2, pyz, __fmul_rn(pyy, uz)), s);
+        s = fmaf(kz * cx, fmaf(pzz, ux, __fmul_rn(uz2, pxz)), s);
+        s = fmaf(kz * cy, fmaf(pzz, uy, __fmul_rn(uz2, pyz)), s);
+        const float c6 = 6.0f * (cx * cy * cz);
+        const float t = fmaf(uz, pxy, fmaf(ux, pyz, __fmul_rn(uy, pxz)));
+        h = __fadd_rn(h, two_products(3.0f, s, c6, t, c6 > 0.0f));
+    }
+    return __fmul_rn(__fmul_rn(d.w, 4.5f), h);
 }
 
 __device__ __forceinline__ bool in_range(int v, int lo, int hi) { return v >= lo && v <= hi; }
@@ -123,10 +146,10 @@ constexpr uint64_t face_list(int axis, int s) {
 template <int Q>
 __device__ __forceinline__ float regularized(const Fields &F, const Dir &d, uint32_t fn, float rho, float ux, float uy,
                                              float uz, float omco) {
-    const float feq = feq_of<Q>(d.cx, d.cy, d.cz, d.w, rho, ux, uy, uz);
-    const float fneq = fneq_of<Q>(d.cx, d.cy, d.cz, d.w, F.pxx[fn], F.pyy[fn], F.pzz[fn], F.pxy[fn], F.pxz[fn],
-                                  F.pyz[fn], F.ux[fn], F.uy[fn], F.uz[fn]);
-    return feq + omco * fneq;
+    const float feq = feq_of<Q>(d, rho, ux, uy, uz);
+    const float fneq = fneq_of<Q>(d, F.pxx[fn], F.pyy[fn], F.pzz[fn], F.pxy[fn], F.pxz[fn], F.pyz[fn], F.ux[fn],
+                                  F.uy[fn], F.uz[fn]);
+    return fmaf(omco, fneq, feq);
 }
 
 // phi and u of the ghost pair (gL, gR) from the fluid cells (bR, bL) they repeat.
