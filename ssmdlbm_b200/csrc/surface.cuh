@@ -16,31 +16,28 @@
 
 namespace ssmd {
 
-// Velocity c and weight of one direction, for code that picks it at run time.
+// Velocity c and weight of one direction.
 struct Dir {
     float cx, cy, cz, w;
     int ix, iy, iz; // the same components as integers
 };
 
-constexpr uint64_t pack_axis(int axis) { // 2 bits per direction: c + 1
-    uint64_t v = 0;
-    for (int q = 0; q < 27; ++q)
-        v |= (uint64_t)((axis == 0 ? cx27(q) : (axis == 1 ? cy27(q) : cz27(q))) + 1) << (2 * q);
-    return v;
+template <int Q>
+__host__ __device__ constexpr Dir dir_of(int q) {
+    return Dir{float(cx27(q)), float(cy27(q)), float(cz27(q)), VS<Q>::w(q), cx27(q), cy27(q), cz27(q)};
 }
 
-template <int Q>
-__device__ __forceinline__ Dir direction(int q) {
-    constexpr uint64_t X = pack_axis(0), Y = pack_axis(1), Z = pack_axis(2);
-    Dir d;
-    d.ix = (int)((X >> (2 * q)) & 3u) - 1;
-    d.iy = (int)((Y >> (2 * q)) & 3u) - 1;
-    d.iz = (int)((Z >> (2 * q)) & 3u) - 1;
-    d.cx = float(d.ix);
-    d.cy = float(d.iy);
-    d.cz = float(d.iz);
-    d.w = q == 0 ? VS<Q>::w(0) : (q <= 6 ? VS<Q>::w1 : (q <= 18 ? VS<Q>::w2 : VS<Q>::w3));
-    return d;
+// Component of a direction picked at run time along `axis`.
+constexpr int axis_of(int axis, int q) { return axis == 0 ? cx27(q) : (axis == 1 ? cy27(q) : cz27(q)); }
+constexpr uint64_t pack_axis(int axis) { // 2 bits per direction: c + 1
+    uint64_t v = 0;
+    for (int q = 0; q < 27; ++q) v |= (uint64_t)(axis_of(axis, q) + 1) << (2 * q);
+    return v;
+}
+template <int AXIS>
+__device__ __forceinline__ int component(int q) {
+    constexpr uint64_t V = pack_axis(AXIS);
+    return (int)((V >> (2 * q)) & 3u) - 1;
 }
 
 // The boundary values' arithmetic is written out, one rounding per operation: a
@@ -71,7 +68,7 @@ __device__ __forceinline__ float feq_of(const Dir &d, float rho, float ux, float
 
 template <int Q, int q>
 __device__ __forceinline__ float feq_dir(float rho, float ux, float uy, float uz) {
-    constexpr Dir d{float(cx27(q)), float(cy27(q)), float(cz27(q)), VS<Q>::w(q), cx27(q), cy27(q), cz27(q)};
+    constexpr Dir d = dir_of<Q>(q);
     return feq_of<Q>(d, rho, ux, uy, uz);
 }
 
@@ -109,29 +106,33 @@ __device__ __forceinline__ float inlet_speed(const Physics &P, unsigned long lon
     return __fmul_rn(P.u_oil, __fadd_rn(1.0f, __fmul_rn(P.noise_amp, n)));
 }
 
-// How the boundary launches are split.  A face has few cells and, with one
-// thread per face cell doing every direction, a launch was ~700 instructions of
+// How the boundary launches are split.  A face has few cells.  With one thread
+// per face cell doing every direction, a launch was ~700 instructions of
 // straight-line code run once by a handful of warps, each direction's loads
 // behind the store of the one before: 4-5 us of fetches and round trips whatever
 // the lattice, 26 us for the x copies, whose every access is a sector of its
-// own (101 x 75 x 203 crossflow, D3Q27 F16_G32: 45 us a step in five launches, 21
-// in three as below; 64 x 64 x 128 jet 5.0 -> 3.0 us).  So every (face cell, population slot) has a thread of its own, the
-// direction is picked at run time (the code is a ninth), and the two faces of an
-// axis share a launch: inflow writes ghost plane 0 and reads plane 1, outflow
-// writes plane n - 1 and reads plane n - 2 (axes with jets have n >= 6), so neither
-// reads what the other writes.  The reference's order (above) is kept by pairs,
-// (water inflow, outflow y) before (oil inflow, outflow z): oil inflow reads
-// fluid cells only and writes plane z = 0, outflow y reads and writes at fluid
-// z, so these two may change places.
+// own.  So
+//  - a jet face cell has three threads, each with one row of up to three
+//    directions (regularized_row), all its loads in flight at once;
+//  - a copied pair has a thread per population slot, the direction picked at run time;
+//  - the two faces of an axis share a launch: inflow writes ghost plane 0 and
+//    reads plane 1, outflow writes plane n - 1 and reads plane n - 2 (axes with jets
+//    have n >= 6), so neither reads what the other writes.
+// us a launch on B200, one thread per face cell -> now: jet faces of 64 x 64 x 128
+// D3Q19 FP32 5.0 -> 3.5, 128 x 128 x 512 D3Q27 FP32 6.6 -> 4.5, 256 x 256 x 1024 D3Q19
+// FP32 5.9 -> 4.6, 24 jets at once 16 -> 12; x copies of a 101 x 75 x 203 crossflow
+// (D3Q27 F16_G32) 25 -> 13, its boundaries altogether 44 in five launches -> 21 in three.
+// The reference's order (above) is kept by pairs, (water inflow, outflow y)
+// before (oil inflow, outflow z): oil inflow reads fluid cells only and writes
+// plane z = 0, outflow y reads and writes at fluid z, so these two may change
+// places.
 constexpr int kFaceX = 32, kFaceY = 4; // a block's face cells
-// population slots of a face (directions that leave it, then the macroscopic fields
-// with the g slot) and of a copy pair (directions with a component along the axis, g,
-// the fields)
+// directions that leave a face; a copied pair has the slots of both, one for g and
+// one for the fields
 template <int Q>
 constexpr int kFaceDirs = Q == 27 ? 9 : 5;
 
 // The directions whose component along `axis` is s (or, s = 0, is not zero), 5 bits each.
-constexpr int axis_of(int axis, int q) { return axis == 0 ? cx27(q) : (axis == 1 ? cy27(q) : cz27(q)); }
 template <int Q>
 constexpr uint64_t face_list(int axis, int s) {
     uint64_t v = 0;
@@ -141,15 +142,48 @@ constexpr uint64_t face_list(int axis, int s) {
     return v;
 }
 
-// Regularized inflow / outflow value of direction d for a ghost cell:
-// f = f_eq(rho_b, u_b) + omco f_neq(Pi(fn), u(fn)) at fluid node fn.
-template <int Q>
-__device__ __forceinline__ float regularized(const Fields &F, const Dir &d, uint32_t fn, float rho, float ux, float uy,
-                                             float uz, float omco) {
-    const float feq = feq_of<Q>(d, rho, ux, uy, uz);
-    const float fneq = fneq_of<Q>(d, F.pxx[fn], F.pyy[fn], F.pzz[fn], F.pxy[fn], F.pxz[fn], F.pyz[fn], F.ux[fn],
-                                  F.uy[fn], F.uz[fn]);
-    return fmaf(omco, fneq, feq);
+// Regularized inflow / outflow values of one row of directions for the ghost cell b
+// of face cell (x, i1), f = f_eq(rho_b, u_b) + omco f_neq(Pi(fn), u(fn)) at fluid
+// node fn: the directions with component S along AXIS (1: y, 2: z) and ROW along
+// the face's second axis.  FLUID: only where fn is a fluid cell (otherwise: inside
+// the lattice).  All loads come before the first store.
+template <int Q, int AXIS, int S, int ROW, bool FLUID, class TF, class TG>
+__device__ __forceinline__ void regularized_row(const StepArgs<TF, TG> &a, int x, int i1, uint32_t b, float rho,
+                                                float ux, float uy, float uz, float omco) {
+    const Geometry &G = a.geo;
+    const Fields &F = a.fld;
+    const int j = AXIS == 1 ? axis_nb(i1 + ROW, G.nz, G.bcz == BC_PERIODIC)
+                            : axis_nb(i1 + ROW, G.ny, G.bcy == BC_PERIODIC);
+    if (j < 0 || (FLUID && !(AXIS == 1 ? in_range(j, G.z_lo, G.z_hi) : in_range(j, G.y_lo, G.y_hi)))) return;
+    const int plane = S > 0 ? 1 : (int)(AXIS == 1 ? G.ny : G.nz) - 2;
+    const uint32_t row = AXIS == 1 ? cell_index(G, 0, plane, j) : cell_index(G, 0, j, plane);
+    float v[3][9];
+    bool ok[3];
+    unroll<0, 3>([&](auto k) {
+        constexpr int K = decltype(k)::value, q = AXIS == 1 ? q27(K - 1, S, ROW) : q27(K - 1, ROW, S);
+        if constexpr (q < Q) {
+            const int xx = axis_nb(x + K - 1, G.nx, G.bcx == BC_PERIODIC);
+            ok[K] = xx >= 0 && (!FLUID || in_range(xx, G.x_lo, G.x_hi));
+            if (ok[K]) {
+                const uint32_t fn = row + (uint32_t)xx;
+                v[K][0] = F.pxx[fn], v[K][1] = F.pyy[fn], v[K][2] = F.pzz[fn];
+                v[K][3] = F.pxy[fn], v[K][4] = F.pxz[fn], v[K][5] = F.pyz[fn];
+                v[K][6] = F.ux[fn], v[K][7] = F.uy[fn], v[K][8] = F.uz[fn];
+            }
+        }
+    });
+    unroll<0, 3>([&](auto k) {
+        constexpr int K = decltype(k)::value, q = AXIS == 1 ? q27(K - 1, S, ROW) : q27(K - 1, ROW, S);
+        if constexpr (q < Q) {
+            if (ok[K]) {
+                constexpr Dir d = dir_of<Q>(q);
+                const float feq = feq_of<Q>(d, rho, ux, uy, uz);
+                const float fneq = fneq_of<Q>(d, v[K][0], v[K][1], v[K][2], v[K][3], v[K][4], v[K][5], v[K][6],
+                                              v[K][7], v[K][8]);
+                Store<TF>::st(a.f_dst + slot(G, q, b), fmaf(omco, fneq, feq));
+            }
+        }
+    });
 }
 
 // phi and u of the ghost pair (gL, gR) from the fluid cells (bR, bL) they repeat.
@@ -167,9 +201,9 @@ __device__ __forceinline__ void copy_ghost_fields(const Fields &F, uint32_t gL, 
     F.uz[gR] = z1;
 }
 
-// Water inflow disc on y = 0 (BoundaryConditions.cuh:36-99).  Thread (x, z), slot k.
-template <int Q, class TF, class TG>
-__device__ __forceinline__ void bc_water_inflow_at(const StepArgs<TF, TG> &a, const int x, const int z, const int k) {
+// Water inflow disc on y = 0 (BoundaryConditions.cuh:36-99).  Thread (x, z), row of directions.
+template <int Q, int ROW, class TF, class TG>
+__device__ __forceinline__ void bc_water_inflow_at(const StepArgs<TF, TG> &a, const int x, const int z) {
     const Geometry &G = a.geo;
     const Physics &P = a.phys;
     if (x >= (int)G.nx || z >= (int)G.nz) return;
@@ -177,27 +211,21 @@ __device__ __forceinline__ void bc_water_inflow_at(const StepArgs<TF, TG> &a, co
     if (dx * dx + dz * dz > P.water_r2) return;
     const uint32_t b = cell_index(G, x, 0, z);
     const float uw = P.u_water;
-    if (k == kFaceDirs<Q>) {
+    // (a node outside the lattice, which the reference reads out of bounds, is left out)
+    regularized_row<Q, 1, 1, ROW, false>(a, x, z, b, 1.0f, 0.0f, uw, 0.0f, P.omco_water);
+    if constexpr (ROW == 0) {
         a.fld.rho[b] = 1.0f;
         a.fld.phi[b] = 0.0f;
         a.fld.ux[b] = 0.0f;
         a.fld.uy[b] = uw;
         a.fld.uz[b] = 0.0f;
         Store<TG>::st(a.g_dst + slot(G, 3, b), 0.0f); // w_3 * phi (1 + 4 u_y) with phi = 0
-        return;
     }
-    const int q = (int)((face_list<Q>(1, 1) >> (5 * k)) & 31u);
-    const Dir d = direction<Q>(q);
-    const int xx = axis_nb(x + d.ix, G.nx, G.bcx == BC_PERIODIC);
-    const int zz = axis_nb(z + d.iz, G.nz, G.bcz == BC_PERIODIC);
-    if (xx < 0 || zz < 0) return; // outside the lattice (the reference reads out of bounds)
-    Store<TF>::st(a.f_dst + slot(G, q, b),
-                  regularized<Q>(a.fld, d, cell_index(G, xx, 1, zz), 1.0f, 0.0f, uw, 0.0f, P.omco_water));
 }
 
-// Oil inflow disc on z = 0 (BoundaryConditions.cuh:101-168).  Thread (x, y), slot k.
-template <int Q, class TF, class TG>
-__device__ __forceinline__ void bc_oil_inflow_at(const StepArgs<TF, TG> &a, const int x, const int y, const int k) {
+// Oil inflow disc on z = 0 (BoundaryConditions.cuh:101-168).  Thread (x, y), row of directions.
+template <int Q, int ROW, class TF, class TG>
+__device__ __forceinline__ void bc_oil_inflow_at(const StepArgs<TF, TG> &a, const int x, const int y) {
     const Geometry &G = a.geo;
     const Physics &P = a.phys;
     if (x >= (int)G.nx || y >= (int)G.ny) return;
@@ -208,79 +236,58 @@ __device__ __forceinline__ void bc_oil_inflow_at(const StepArgs<TF, TG> &a, cons
     if (P.noise_amp != 0.0f) {
         uin = inlet_speed(P, a.status->step, b);
     }
-    if (k == kFaceDirs<Q>) {
+    regularized_row<Q, 2, 1, ROW, true>(a, x, y, b, 1.0f, 0.0f, 0.0f, uin, P.omco_oil);
+    if constexpr (ROW == 0) {
         a.fld.rho[b] = 1.0f;
         a.fld.phi[b] = 1.0f;
         a.fld.ux[b] = 0.0f;
         a.fld.uy[b] = 0.0f;
         a.fld.uz[b] = uin;
         Store<TG>::st(a.g_dst + slot(G, 5, b), kW7_1 * 1.0f * (1.0f + 4.0f * uin));
-        return;
     }
-    const int q = (int)((face_list<Q>(2, 1) >> (5 * k)) & 31u);
-    const Dir d = direction<Q>(q);
-    const int xx = axis_nb(x + d.ix, G.nx, G.bcx == BC_PERIODIC);
-    const int yy = axis_nb(y + d.iy, G.ny, G.bcy == BC_PERIODIC);
-    if (xx < 0 || yy < 0 || !in_range(xx, G.x_lo, G.x_hi) || !in_range(yy, G.y_lo, G.y_hi)) return;
-    Store<TF>::st(a.f_dst + slot(G, q, b),
-                  regularized<Q>(a.fld, d, cell_index(G, xx, yy, 1), 1.0f, 0.0f, 0.0f, uin, P.omco_oil));
 }
 
-// Outflow on y = ny-1 (BoundaryConditions.cuh:170-233).  Thread (x, z), slot k.
-template <int Q, class TF, class TG>
-__device__ __forceinline__ void bc_outflow_y_at(const StepArgs<TF, TG> &a, const int x, const int z, const int k) {
+// Outflow on y = ny-1 (BoundaryConditions.cuh:170-233).  Thread (x, z), row of directions.
+template <int Q, int ROW, class TF, class TG>
+__device__ __forceinline__ void bc_outflow_y_at(const StepArgs<TF, TG> &a, const int x, const int z) {
     const Geometry &G = a.geo;
     if (!in_range(x, G.x_lo, G.x_hi) || !in_range(z, G.z_lo, G.z_hi)) return;
     const uint32_t b = cell_index(G, x, G.ny - 1, z);
     const uint32_t i1 = cell_index(G, x, G.ny - 2, z);
     const Fields &F = a.fld;
     const float ux = F.ux[i1], uy = F.uy[i1], uz = F.uz[i1], rho = F.rho[i1];
-    if (k == kFaceDirs<Q>) {
-        const float phi = F.phi[i1];
+    const float phi = ROW == 0 ? F.phi[i1] : 0.f;
+    regularized_row<Q, 1, -1, ROW, true>(a, x, z, b, rho, ux, uy, uz, a.phys.omco_ref);
+    if constexpr (ROW == 0) {
         F.rho[b] = rho;
         F.phi[b] = phi;
         F.ux[b] = ux;
         F.uy[b] = uy;
         F.uz[b] = uz;
         Store<TG>::st(a.g_dst + slot(G, 4, b), kW7_1 * phi * (1.0f - 4.0f * uy));
-        return;
     }
-    const int q = (int)((face_list<Q>(1, -1) >> (5 * k)) & 31u);
-    const Dir d = direction<Q>(q);
-    const int xx = axis_nb(x + d.ix, G.nx, G.bcx == BC_PERIODIC);
-    const int zz = axis_nb(z + d.iz, G.nz, G.bcz == BC_PERIODIC);
-    if (xx < 0 || zz < 0 || !in_range(xx, G.x_lo, G.x_hi) || !in_range(zz, G.z_lo, G.z_hi)) return;
-    Store<TF>::st(a.f_dst + slot(G, q, b),
-                  regularized<Q>(F, d, cell_index(G, xx, G.ny - 2, zz), rho, ux, uy, uz, a.phys.omco_ref));
 }
 
-// Outflow on z = nz-1 (BoundaryConditions.cuh:235-293).  Thread (x, y), slot k.
-template <int Q, class TF, class TG>
-__device__ __forceinline__ void bc_outflow_z_at(const StepArgs<TF, TG> &a, const int x, const int y, const int k) {
+// Outflow on z = nz-1 (BoundaryConditions.cuh:235-293).  Thread (x, y), row of directions.
+template <int Q, int ROW, class TF, class TG>
+__device__ __forceinline__ void bc_outflow_z_at(const StepArgs<TF, TG> &a, const int x, const int y) {
     const Geometry &G = a.geo;
     if (!in_range(x, G.x_lo, G.x_hi) || !in_range(y, G.y_lo, G.y_hi)) return;
     const uint32_t b = cell_index(G, x, y, G.nz - 1);
     const uint32_t i1 = cell_index(G, x, y, G.nz - 2);
     const Fields &F = a.fld;
     const float ux = F.ux[i1], uy = F.uy[i1], uz = F.uz[i1], rho = F.rho[i1];
-    if (k == kFaceDirs<Q>) {
-        const float phi = F.phi[i1];
+    const float phi = ROW == 0 ? F.phi[i1] : 0.f;
+    // no fluid-range check here, as in the reference (ghost nodes allowed)
+    regularized_row<Q, 2, -1, ROW, false>(a, x, y, b, rho, ux, uy, uz, a.phys.omco_ref);
+    if constexpr (ROW == 0) {
         F.rho[b] = rho;
         F.phi[b] = phi;
         F.ux[b] = ux;
         F.uy[b] = uy;
         F.uz[b] = uz;
         Store<TG>::st(a.g_dst + slot(G, 6, b), kW7_1 * phi * (1.0f - 4.0f * uz));
-        return;
     }
-    const int q = (int)((face_list<Q>(2, -1) >> (5 * k)) & 31u);
-    const Dir d = direction<Q>(q);
-    // no fluid-range check here, as in the reference (ghost nodes allowed)
-    const int xx = axis_nb(x + d.ix, G.nx, G.bcx == BC_PERIODIC);
-    const int yy = axis_nb(y + d.iy, G.ny, G.bcy == BC_PERIODIC);
-    if (xx < 0 || yy < 0) return;
-    Store<TF>::st(a.f_dst + slot(G, q, b),
-                  regularized<Q>(F, d, cell_index(G, xx, yy, G.nz - 2), rho, ux, uy, uz, a.phys.omco_ref));
 }
 
 // Copy-periodic x (BoundaryConditions.cuh:295-349).  Thread (y, z), all y, z; slot k.
@@ -296,8 +303,8 @@ __device__ __forceinline__ void bc_copy_x_at(const StepArgs<TF, TG> &a, const in
     constexpr int D = kFaceDirs<Q>;
     if (k < 2 * D) {
         const int q = (int)(((k < D ? face_list<Q>(0, 1) : face_list<Q>(0, -1)) >> (5 * (k < D ? k : k - D))) & 31u);
-        const Dir d = direction<Q>(q);
-        const int hy = axis_nb(y - d.iy, G.ny, G.bcy == BC_PERIODIC), hz = axis_nb(z - d.iz, G.nz, G.bcz == BC_PERIODIC);
+        const int hy = axis_nb(y - component<1>(q), G.ny, G.bcy == BC_PERIODIC);
+        const int hz = axis_nb(z - component<2>(q), G.nz, G.bcz == BC_PERIODIC);
         if (hy < 0 || hz < 0) return;
         const int to = k < D ? 0 : nx - 1;
         const int from = k < D ? nx - 3 : 2;
@@ -328,8 +335,8 @@ __device__ __forceinline__ void bc_copy_y_at(const StepArgs<TF, TG> &a, const in
     constexpr int D = kFaceDirs<Q>;
     if (k < 2 * D) {
         const int q = (int)(((k < D ? face_list<Q>(1, 1) : face_list<Q>(1, -1)) >> (5 * (k < D ? k : k - D))) & 31u);
-        const Dir d = direction<Q>(q);
-        const int hx = axis_nb(x - d.ix, G.nx, G.bcx == BC_PERIODIC), hz = axis_nb(z - d.iz, G.nz, G.bcz == BC_PERIODIC);
+        const int hx = axis_nb(x - component<0>(q), G.nx, G.bcx == BC_PERIODIC);
+        const int hz = axis_nb(z - component<2>(q), G.nz, G.bcz == BC_PERIODIC);
         if (hx < 0 || hz < 0) return;
         const int to = k < D ? 0 : ny - 1;
         const int from = k < D ? ny - 3 : 2;
@@ -352,21 +359,24 @@ __device__ __forceinline__ void bc_copy_y_at(const StepArgs<TF, TG> &a, const in
 // ---- launches ------------------------------------------------------------------
 enum : int { BK_JET_Y = 0, BK_JET_Z, BK_COPY_X, BK_COPY_Y };
 
-// Faces of a launch, and slots of each.
+// Faces of a launch, and threads per cell of each: the rows of directions of a jet
+// face, the slots of a copied pair.
 template <int K>
 constexpr int kFaces = K == BK_JET_Y || K == BK_JET_Z ? 2 : 1;
 template <int Q, int K>
-constexpr int kSlots = K == BK_JET_Y || K == BK_JET_Z ? kFaceDirs<Q> + 1 : 2 * kFaceDirs<Q> + 2;
+constexpr int kSlots = K == BK_JET_Y || K == BK_JET_Z ? 3 : 2 * kFaceDirs<Q> + 2;
 
 // Grid of one boundary launch over faces of at most n0 x n1 cells of `count`
 // lattices: blocks of kFaceX x kFaceY face cells, blockIdx.x the tiles along the
-// first axis times the slots of the faces.  (Several slots per thread in a loop, so
-// that all blocks of a large face are resident at once, lost to the round trips
-// that then follow one another: 256 x 256 face 5.6 -> 7.4 us, crossflow 21 -> 26.  The one
-// loss: three 128 x 128 x 512 D3Q27 FP32 jets on streams of their own, whose bulk blocks
-// fill every SM, take 484 us for each step instead of 480; one alone in a replayed graph
-// takes 450 instead of 456.  One thread per cell there brought the 484 to 481 and the 450
-// to 459.)
+// first axis times the slots of the faces.
+// A thread per (cell, slot) on jet faces too is a little shorter on an idle device
+// (the launches above: 3.2, 3.9, 5.5, 16 us) but 2560 blocks for a 128 x 128 face, and
+// among other lattices' kernels, which fill every SM, their instructions and places
+// count: three 128 x 128 x 512 D3Q27 FP32 jets on their own streams took 467 us a step
+// each, with rows 464, with one thread per cell 464; one alone in a replayed graph 455.5,
+// 456.7 and 459.3.  All inflow rows in one thread: 38.4 instead of 37.1 us a step on 64 x
+// 64 x 128.  For the copies, several slots per thread in a loop lost to the round trips
+// that follow one another (crossflow 21 -> 26 us).
 template <int Q, int K>
 inline dim3 face_grid(uint32_t n0, uint32_t n1, unsigned count = 1) {
     return dim3((n0 + kFaceX - 1) / kFaceX * (kFaces<K> * kSlots<Q, K>), (n1 + kFaceY - 1) / kFaceY, count);
@@ -379,15 +389,26 @@ __device__ __forceinline__ void bc_face(const StepArgs<TF, TG> &a) {
     const int s = (int)blockIdx.x / tiles; // slot of the first face, then of the second
     const int i0 = ((int)blockIdx.x - s * tiles) * kFaceX + (int)threadIdx.x;
     const int i1 = (int)blockIdx.y * kFaceY + (int)threadIdx.y;
-    constexpr int N = kSlots<Q, K>;
     if constexpr (K == BK_JET_Y) {
         if (G.bcy != BC_JET) return;
-        if (s < N) bc_water_inflow_at<Q>(a, i0, i1, s);
-        else bc_outflow_y_at<Q>(a, i0, i1, s - N);
+        switch (s) {
+        case 0: bc_water_inflow_at<Q, -1>(a, i0, i1); break;
+        case 1: bc_water_inflow_at<Q, 0>(a, i0, i1); break;
+        case 2: bc_water_inflow_at<Q, 1>(a, i0, i1); break;
+        case 3: bc_outflow_y_at<Q, -1>(a, i0, i1); break;
+        case 4: bc_outflow_y_at<Q, 0>(a, i0, i1); break;
+        default: bc_outflow_y_at<Q, 1>(a, i0, i1); break;
+        }
     } else if constexpr (K == BK_JET_Z) {
         if (G.bcz != BC_JET) return;
-        if (s < N) bc_oil_inflow_at<Q>(a, i0, i1, s);
-        else bc_outflow_z_at<Q>(a, i0, i1, s - N);
+        switch (s) {
+        case 0: bc_oil_inflow_at<Q, -1>(a, i0, i1); break;
+        case 1: bc_oil_inflow_at<Q, 0>(a, i0, i1); break;
+        case 2: bc_oil_inflow_at<Q, 1>(a, i0, i1); break;
+        case 3: bc_outflow_z_at<Q, -1>(a, i0, i1); break;
+        case 4: bc_outflow_z_at<Q, 0>(a, i0, i1); break;
+        default: bc_outflow_z_at<Q, 1>(a, i0, i1); break;
+        }
     } else if constexpr (K == BK_COPY_X) {
         if (G.bcx == BC_COPY) bc_copy_x_at<Q>(a, i0, i1, s);
     } else {
