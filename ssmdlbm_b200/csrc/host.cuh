@@ -167,7 +167,9 @@ static __global__ void averages_kernel(Geometry G, Fields F, Averages A, DeviceS
     __syncthreads(); // every thread has read avg_t
     if (threadIdx.x == 0) {
         const unsigned blocks = gridDim.x * gridDim.y;
+        __threadfence(); // the block's reads before its ticket
         if (atomicAdd(&status->work_next, 1u) == blocks - 1u) { // every block has
+            __threadfence(); // the tickets before the update
             status->work_next = 0u;
             status->avg_t += 1u;
         }
