@@ -471,7 +471,10 @@ int ssmd_derived_update(const ssmd_params *p, const LBMFields *fields, uint32_t 
  *     is not NULL, ssmd_mlp_average(avg, net, decay); two kernels.  A row index
  *     outside [0, n_rows) contributes nothing and sets bit 1 of the status.
  *   ssmd_mlp_status: bit 0 set when an MMA wait timed out (the CTA aborted), bit 1
- *     when a training step met a row index out of range.
+ *     when a training step met a row index out of range.  A CTA that aborted has
+ *     no gradient: ssmd_mlp_grad_ws and ssmd_mlp_train_step then leave NaN in grad and
+ *     loss (ssmd_mlp_grad in loss), and the training step leaves net, m, v and avg
+ *     as they were.
  * Features (ssmd_closure_features), per cell, from rho, ux, uy, uz, phi with
  * central differences (periodic axes wrap, others clamp at the faces):
  *   phi, 4 phi (1 - phi), |grad phi|, laplacian phi, |S| = sqrt(2 S:S),

@@ -44,6 +44,7 @@
 
 #include <algorithm>
 
+#include "adam.cuh"
 #include "closure.cuh"
 #include "host.cuh"
 #include "umma.cuh"
@@ -78,7 +79,6 @@ constexpr uint32_t col_r() { return MODE == kTrain ? 128u : 0u; }
 constexpr uint32_t cZ1 = 0, cDH1 = 192, cG1 = 256, cG2 = 336;
 constexpr int kGB = 2 * kH + 16;   // columns of the gradient tile: dZ1, dZ2, dR (2 of 16)
 constexpr uint64_t kMmaWaitNs = 1000000000ull;
-constexpr int kMaxGradCtas = 256; // rows of the deterministic gradient workspace
 
 // shared-memory map (bytes from an aligned base: 1024 bytes for training,
 // 128 for inference; the no-swizzle operand layout needs 16).  Training, all
@@ -725,6 +725,9 @@ __global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpAr
         } else if ((tid & 31) == 0 && grp == 0) {
             atomicAdd(a.loss, (double)l / (double)n);
         }
+    } else if (tid == 0) { // no sums: the gradient of this call is not to be used
+        if (a.partials) a.partials[(size_t)blockIdx.x * (kParams + 1) + kParams] = aborted_mark();
+        else atomicAdd(a.loss, (double)aborted_mark());
     }
 
     // ---- tear-down: every TMEM read is complete before the warp frees it
@@ -732,72 +735,6 @@ __global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpAr
     __syncthreads();
     if (!ok && tid == 0) atomicOr(&g_mlp_status, 1u);
     if (warp == 0) umma::tmem_dealloc(tmem, tmem_cols<kTrain>());
-}
-
-__device__ __forceinline__ void adam_update(float &p, float gi, float &m, float &v, float lr, float beta1, float beta2,
-                                            float eps, float corr1, float corr2) {
-    // (explicit fma: the kernels that share this round alike)
-    m = fmaf(1.0f - beta1, gi, beta1 * m);
-    v = fmaf((1.0f - beta2) * gi, gi, beta2 * v);
-    p -= lr * (m / corr1) / (sqrtf(v / corr2) + eps);
-}
-__device__ __forceinline__ float average_update(float avg, float p, float decay) {
-    return fmaf(decay, avg - p, p); // decay avg + (1 - decay) p
-}
-
-// Adam step and weight average that follow a gradient (m null: none; avg null: none).
-struct AdamArgs {
-    float *net, *m, *v, *avg;
-    float lr, beta1, beta2, eps, corr1, corr2, decay;
-};
-
-// Deterministic reduction of the per-CTA gradient rows, column k summed over the
-// CTAs in CTA order (FP32, like the atomic path; the loss column in FP64), then
-// the Adam step and the average on it.  A block takes 32 columns: its
-// 8 warps bring the rows into shared memory, all in flight at once, and one
-// warp adds them.  (A thread per column that loaded its rows one after the other:
-// 8.5 us, and 4 us more for Adam and the average in launches of their own; now 4.6 us
-// for all three.)
-constexpr int kSumThreads = 256;
-__global__ void __launch_bounds__(kSumThreads)
-    grad_sum_kernel(const float *__restrict__ partials, int ctas, int64_t n, float *__restrict__ grad,
-                    double *__restrict__ loss, const AdamArgs ad) {
-    __shared__ float s[kMaxGradCtas][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int k = blockIdx.x * 32 + lane;
-    // Adam's operands are on their way while the rows come in
-    const bool step = warp == 0 && k < kParams;
-    const float m0 = step && ad.m ? ad.m[k] : 0.f, v0 = step && ad.m ? ad.v[k] : 0.f;
-    const float p0 = step && ad.net ? ad.net[k] : 0.f, a0 = step && ad.avg ? ad.avg[k] : 0.f;
-    float row[kMaxGradCtas / (kSumThreads / 32)];
-#pragma unroll
-    for (int i = 0; i < kMaxGradCtas / (kSumThreads / 32); ++i) {
-        const int b = warp + i * (kSumThreads / 32);
-        row[i] = b < ctas && k <= kParams ? __ldg(partials + (size_t)b * (kParams + 1) + k) : 0.f;
-    }
-#pragma unroll
-    for (int i = 0; i < kMaxGradCtas / (kSumThreads / 32); ++i) s[warp + i * (kSumThreads / 32)][lane] = row[i];
-    __syncthreads();
-    if (warp != 0) return;
-    if (k < kParams) {
-        float g = 0.f;
-#pragma unroll 8
-        for (int b = 0; b < ctas; ++b) g += s[b][lane];
-        grad[k] = g;
-        float p = p0;
-        if (ad.m) {
-            float m = m0, v = v0;
-            adam_update(p, g, m, v, ad.lr, ad.beta1, ad.beta2, ad.eps, ad.corr1, ad.corr2);
-            ad.net[k] = p;
-            ad.m[k] = m;
-            ad.v[k] = v;
-        }
-        if (ad.avg) ad.avg[k] = average_update(a0, p, ad.decay);
-    } else if (k == kParams) {
-        double l = 0.0;
-        for (int b = 0; b < ctas; ++b) l += (double)s[b][lane];
-        *loss = l / (double)n;
-    }
 }
 
 __global__ void adam_kernel(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
@@ -883,7 +820,7 @@ int launch(MlpArgs a, cudaStream_t st, int max_ctas = 0, const AdamArgs &ad = Ad
     kernel_of<MODE>()<<<blocks, kThreadsOf<MODE>, smem, st>>>(a);
     if (int e = cuda_check(cudaGetLastError(), "mlp launch")) return e;
     if (MODE == kTrain && a.partials) {
-        grad_sum_kernel<<<(kParams + 1 + 31) / 32, kSumThreads, 0, st>>>(a.partials, (int)blocks, a.n, a.grad, a.loss, ad);
+        grad_sum_kernel<kParams><<<(kParams + 1 + 31) / 32, kSumThreads, 0, st>>>(a.partials, (int)blocks, a.n, a.grad, a.loss, ad);
         return cuda_check(cudaGetLastError(), "gradient sum launch");
     }
     return SSMD_OK;
