@@ -6,13 +6,13 @@
 // tanh from the SFU (tanh.approx.f32, absolute error about 2^-11, below the
 // bf16 rounding of the hidden activations that follows), features
 // standardised by stored mean / inverse std, outputs p = scale * r + offset
-// with r the last layer's raw output.  A persistent CTA of 128 threads loops
-// over tiles of 128 cells (thread i <-> cell row i of the tile), weights
-// staged once per CTA:
+// with r the last layer's raw output.  A persistent CTA loops over tiles of 128
+// cells, weights staged once per CTA; inference: 128 threads, thread i <-> cell row i
+// of the tile; training: 512 threads, four per row (mlp_train_kernel):
 //   X [128 x 16] (bf16, K padded 12 -> 16)   z1 = X W1^T      (tcgen05, N = 64, K = 16)
 //   H1 = gelu(z1 + b1) [128 x 64] bf16        z2 = H1 W2^T     (4 MMAs of K = 16)
 //   H2 = gelu(z2 + b2) [128 x 64] bf16        r  = H2 W3^T     (N padded 2 -> 16)
-// The epilogues read the accumulators back with tcgen05.ld (the next 16
+// The epilogues read the accumulators back with tcgen05.ld (inference: the next 16
 // columns in flight while the current 16 are processed), add the bias,
 // apply GELU on pairs of columns with packed FP32 arithmetic (fma.rn.f32x2
 // and friends, sm_100) and write the next layer's bf16 operand.  Inference
@@ -37,8 +37,9 @@
 // ones in X) in TMEM across the CTA's tiles; they run while the next tile
 // begins.  The CTA's sums are then either added across CTAs with
 // atomics (ssmd_mlp_grad) or written as one row per CTA and summed in CTA
-// order by a second kernel (ssmd_mlp_grad_ws: the same bits on every run).  Every wait on an MMA is bounded: on timeout
-// the CTA records bit 0 of the status word, frees its TMEM and returns.
+// order by a second kernel (ssmd_mlp_grad_ws: the same bits on every run).  Every
+// wait on an MMA is bounded: on timeout the CTA records bit 0 of the status word,
+// frees its TMEM and returns.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -97,6 +98,8 @@ constexpr uint32_t sXT = 0, kXBytes = kRows * kK1 * 2, sHH = 2 * kXBytes, sDZ = 
                    sW1T = sDZ + kRows * kGB * 2, sW3T = sW1T + kH * kK1 * 2, sW2T = sW3T + kN3 * kH * 2,
                    sDY = sW2T + kH * kH * 2;
 constexpr uint32_t kXGroup = kK1 / 8 * 128, kHGroup = 2 * kH / 8 * 128, kDGroup = kGB / 8 * 128; // a row group's bytes
+// (the last K step's second row group of the second X buffer, and 128 columns from there)
+static_assert(kXBytes + (kRows / 8 - 1) * kXGroup + 128 / 8 * 128 <= sDZ, "G2's reads past X stay inside X and HH");
 template <int MODE>
 struct Layout {
     static constexpr bool T = MODE == kTrain;
@@ -430,11 +433,12 @@ struct TrainRow {
 // kernel is a chain of MMA round trips and epilogues per tile; with one thread
 // per row (4 warps per SM, one per scheduler) the epilogues' ~5000 instructions
 // ran at the latency of one warp: 15 us a tile, 62 us for 65 536 rows; with four
-// threads per row 40, the gather included, and 28 with the gradient MMAs reading row-wise
-// tiles (see the shared-memory map) and a row's index loaded a tile ahead of the row.  The rows of a mini-batch are read through their
-// indices (a.rows), the next tile's while this one's layers run: gathering them first took
-// three launches and 50 us of the 128 us step.  Every value and every sum is in
-// the order of one thread per row: the same bits.
+// threads per row 40, the gather included, and 28 with the gradient MMAs reading
+// row-wise tiles (see the shared-memory map) and a row's index loaded a tile ahead of
+// the row.  The rows of a mini-batch are read through their indices (a.rows), the
+// next tile's while this one's layers run: gathering them first took three launches
+// and 50 us of the 128 us step.  Every value and every sum is in the order of one
+// thread per row: the same bits.
 __global__ void __launch_bounds__(kThreadsTrain, 1) mlp_train_kernel(const MlpArgs a) {
     using L = Layout<kTrain>;
     extern __shared__ unsigned char smem_raw[];
@@ -807,7 +811,8 @@ int launch_shape(size_t smem, int &per_sm, int &sms) {
 
 template <int MODE>
 int launch(MlpArgs a, cudaStream_t st, int max_ctas = 0, const AdamArgs &ad = AdamArgs{}) {
-    // training: one CTA per SM (its 256 TMEM columns and ~120 KB of shared memory)
+    // training: one CTA per SM (it allocates all 512 TMEM columns; 120 KB of shared
+    // memory keep a second one away, whose allocation would wait for the first to end)
     const size_t smem = MODE == kTrain ? (Layout<MODE>::bytes > (size_t)120 * 1024 ? Layout<MODE>::bytes
                                                                                      : (size_t)120 * 1024)
                                        : Layout<MODE>::bytes;
@@ -820,7 +825,8 @@ int launch(MlpArgs a, cudaStream_t st, int max_ctas = 0, const AdamArgs &ad = Ad
     kernel_of<MODE>()<<<blocks, kThreadsOf<MODE>, smem, st>>>(a);
     if (int e = cuda_check(cudaGetLastError(), "mlp launch")) return e;
     if (MODE == kTrain && a.partials) {
-        grad_sum_kernel<kParams><<<(kParams + 1 + 31) / 32, kSumThreads, 0, st>>>(a.partials, (int)blocks, a.n, a.grad, a.loss, ad);
+        grad_sum_kernel<kParams><<<(kParams + 1 + 31) / 32, kSumThreads, 0, st>>>(a.partials, (int)blocks, a.n, a.grad,
+                                                                                 a.loss, ad);
         return cuda_check(cudaGetLastError(), "gradient sum launch");
     }
     return SSMD_OK;
