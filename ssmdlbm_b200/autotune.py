@@ -19,7 +19,7 @@ import os
 
 from . import _lib
 
-# 0: the library's own choice (a makespan model of the block scheduling, 8-64 planes)
+# 0: the library's own choice (a makespan model of the block scheduling, 8-64 planes; 2-8 on small lattices)
 CANDIDATE_TILE_Z = (0, 12, 16, 20, 24, 28, 32, 48, 56, 64)
 
 

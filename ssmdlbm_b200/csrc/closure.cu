@@ -62,9 +62,10 @@ __device__ __forceinline__ float2 pair_at(const float *__restrict__ a, uint32_t 
     return make_float2(__ldg(a + c), __ldg(a + c + 1));
 }
 
-__global__ void __launch_bounds__(256, 3) filter_kernel(Grid fg, Grid cg, const float *__restrict__ rho, const float *__restrict__ ux,
-                              const float *__restrict__ uy, const float *__restrict__ uz, const float *__restrict__ phi,
-                              float *__restrict__ coarse, float *__restrict__ tau, float *__restrict__ area) {
+__global__ void __launch_bounds__(256, 3)
+    filter_kernel(Grid fg, Grid cg, const float *__restrict__ rho, const float *__restrict__ ux,
+                  const float *__restrict__ uy, const float *__restrict__ uz, const float *__restrict__ phi,
+                  float *__restrict__ coarse, float *__restrict__ tau, float *__restrict__ area) {
     const uint32_t cells = (uint32_t)cg.nx * cg.ny * cg.nz;
     const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (t >= cells) return;
