@@ -112,16 +112,17 @@ struct Bulk {
     // PXY folded into the coordinate arithmetic too, for 16-bit f, which is
     // bound by instruction issue (128 x 128 x 512 jet: D3Q27 FP16 424 -> 409, BF16
     // 423 -> 410, F16_G32 418 -> 405, D3Q19 FP16 365 -> 348, F16_G32 352 -> 338
-    // us), although D3Q27 spills with it (112 bytes FP16 and BF16, 120 F16_G32; none
-    // without): the compiler hoists more out of the plane loop.  FP32 f, bound by
-    // load latency, loses by the same hoisting (D3Q27 456 -> 479, D3Q19 379 -> 388).
+    // us).  D3Q27 spills with it (112 bytes FP16 and BF16, 120 F16_G32), outside the
+    // plane loop: 11 local loads and stores per warp and launch, 0.04 % of its
+    // instructions.  FP32 f, bound by load latency, loses by it: the compiler hoists
+    // more out of the plane loop and spills there (D3Q27 456 -> 479, D3Q19 379 -> 388).
     static constexpr bool kConstXY = PXY && sizeof(TF) == 2;
     // The prologue's phi planes two at a time (fill_phi_pair): shorter for the
     // short columns of small lattices (64 x 64 x 128 jet, D3Q19 FP32: 42.7 -> 41.0
     // us a step; 101 x 75 x 203 crossflow, D3Q27 F16_G32: 181 -> 177).  Off for D3Q27
-    // with PXY, whose plane loop has no register left: what the paired
-    // prologue adds comes on top of the spills above (128 x 128 x 512 jet, with it: BF16
-    // 412 -> 421, F16_G32 408 -> 416, FP32 462 -> 465)
+    // with PXY, where it measured slower (128 x 128 x 512 jet, with it: BF16 412 -> 421,
+    // F16_G32 408 -> 416, FP32 462 -> 465): the plane loop after it is then compiled
+    // another way.  A line by instantiation, as the compiler's choice is.
     static constexpr bool kPairPrologue = Q == 19 || !PXY;
     static __device__ __forceinline__ bool per_x(const Geometry &G) { return kConstXY || G.bcx == BC_PERIODIC; }
     static __device__ __forceinline__ bool per_y(const Geometry &G) { return kConstXY || G.bcy == BC_PERIODIC; }

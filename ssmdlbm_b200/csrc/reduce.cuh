@@ -26,9 +26,10 @@ __device__ __forceinline__ double warp_fold(int k, double v) {
 // kRedPlanes z planes, so a cell costs no division and its loads (the five
 // fields and seven populations) are coalesced and independent of the plane
 // before.  The largest speed is kept squared (sqrt is monotonic and correctly
-// rounded: the same bits).  One cell per thread in linear order, its coordinates
-// from two divisions and a FP64 square root per cell, took 228 us on 128 x 128 x 512 cells (FP32
-// g); this takes 82, at 76 % of the measured copy bandwidth.
+// rounded: the same bits).  On 128 x 128 x 512 cells (FP32 g: 403 MB; caches flushed
+// before the launch) 73 us, 85 % of the measured copy bandwidth; one cell per thread
+// in linear order, its coordinates from two divisions and a FP64 square root per
+// cell, took 224.
 constexpr int kRedPlanes = 16;
 
 template <class TG>
@@ -96,8 +97,8 @@ __global__ void __launch_bounds__(kRedThreads) reduce_pass1(Geometry G, Fields F
     }
 }
 
-// Pass 2: warp k folds value k's partials (one block; 7.7 us as a tree over shared
-// memory, 3.8 now).
+// Pass 2: warp k folds value k's partials (one block; 9.3 us as a tree over shared
+// memory, 5.0 now, caches flushed).
 constexpr int kFoldThreads = 32 * kRedVals;
 static __global__ void __launch_bounds__(kFoldThreads) reduce_pass2(const double *partials, int nparts,
                                                                     double *out) {
